@@ -17,6 +17,13 @@ __device__ __forceinline__ bool test_bit(const uint32_t* bm, uint32_t v) {
   return (__ldg(bm + (v >> 5)) >> (v & 31)) & 1u;
 }
 
+// What a functor's commit reads of its destination (raw 32-bit words):
+// commit(d, acc) is commit_apply(d, commit_load(d), acc), split so that a
+// caller can issue the loads of several destinations before it needs any.
+struct CommitIn {
+  uint32_t a, b;
+};
+
 template <class T>
 __device__ __forceinline__ T warp_sum(T v) {
 #pragma unroll

@@ -142,6 +142,12 @@ struct gg_graph_s {
   gg::SegIndex seg[2];       // row structure of the pulled stream, same indexing
   uint64_t m_pad = 0;        // edge arrays hold m_pad entries (zero padded)
   gg::TileSet coo_tiles;
+  // work items of the direct-load COO pulls: two uint4 each, the tile and
+  // {first 256-edge block, blocks, items of the tile, slab word of the tile};
+  // a tile shared by several items combines their sums in its slab
+  uint4* d_coo_items = nullptr;
+  uint32_t coo_item_count = 0;
+  uint32_t* d_coo_slab = nullptr;  // all zero between launches
   uint2* d_coo_gaps = nullptr;  // {first, count} of the destination ranges outside every COO tile
   uint32_t coo_gap_count = 0;
   bool has_coo = false;
@@ -239,6 +245,9 @@ struct PullParams {
   unsigned long long* stats;   // [0] count [1] out-degree sum
   unsigned long long* err;
   uint32_t tv;                 // widest tile of the tile set
+  const uint4* items;          // work items of the COO tiles (see gg_graph_s::d_coo_items)
+  uint32_t nitems;
+  uint32_t* slab;
 };
 
 // tv: the widest tile of the tile set (its accumulators and flags are sized by it)
@@ -509,6 +518,7 @@ struct finishes<F, decltype((void)F::kFinish)> {
 
 constexpr int kCooWarps = 8;
 constexpr int kCooThreads = kCooWarps * 32;
+constexpr uint64_t kCooItemMinEdges = 4096;  // fewest edges a tile is cut into (build_coo_items)
 
 __host__ __device__ constexpr size_t coo_w_stage_bytes(bool hw) {
   return (size_t)kSegBlock * 4 + (size_t)kSegBlock * 2 + (hw ? (size_t)kSegBlock * 4 : 0);
@@ -535,8 +545,15 @@ __host__ __device__ constexpr size_t coo_w_smem_bytes(bool hw, int stages, int v
 // shuffles before the shared-memory accumulation, so a destination appears in
 // at most one accumulation per block (instead of one per lane it spans, all
 // on one address).
-// The pull as a device function, so that a persistent loop kernel can run it
-// once per iteration (k_pull_coo_w is one call of it).
+// The merging kernels (MERGE) take their work as items: a tile, or a run of
+// 256-edge blocks of one.  What bounds the pull is the L1/LSU pipe of the SMs
+// that still have edges: with one CTA per tile, an R-MAT hub tile (up to
+// tile_edges edges) outlasts every other CTA (R-MAT-22, 2^18-edge tiles, 65M
+// edges on 592 resident CTAs: 110K edges per CTA, 255K in the largest tile).
+// A tile's items add their sums to its slab in global memory (encoded so that
+// zero is the identity of every functor) and the item that arrives last takes
+// the totals back, clears the slab and commits, so that every destination is
+// still committed once.
 // F::gather_pol (a gather that takes an L2 eviction policy), when declared
 template <class F, class = void>
 struct has_gather_pol : std::false_type {};
@@ -567,7 +584,7 @@ __device__ __forceinline__ void pull_coo_w_run(const PullParams& p, const F& f) 
   __shared__ uint32_t s_tile;
   __shared__ unsigned long long s_red[2][kCooWarps];
   __shared__ double s_l1[kFin ? kCooWarps : 1];
-  __shared__ int s_fail;
+  __shared__ int s_fail, s_last;
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   uint64_t* wbar = bars + warp * (STAGES > 0 ? STAGES : 1);
@@ -601,8 +618,9 @@ __device__ __forceinline__ void pull_coo_w_run(const PullParams& p, const F& f) 
     if (tid == 0) s_tile = (uint32_t)atomicAdd(p.tile_counter, 1ull);
     __syncthreads();
     const uint32_t t = s_tile;
-    if (t >= p.ntiles || s_fail) break;
-    const uint4 td = p.tiles[t];
+    if (t >= (MERGE ? p.nitems : p.ntiles) || s_fail) break;
+    const uint4 td = MERGE ? p.items[2 * t] : p.tiles[t];
+    const uint4 part = MERGE ? p.items[2 * t + 1] : make_uint4(0, 0, 1, 0);
     const uint32_t v0 = td.x, nv = td.y, e0 = td.z, ne = td.w;  // e0, ne multiples of 8
     for (uint32_t i = tid; i < nv; i += kCooThreads) {
       s_acc[i] = F::identity();
@@ -610,7 +628,7 @@ __device__ __forceinline__ void pull_coo_w_run(const PullParams& p, const F& f) 
       if (!F::kCondTrue) s_cond[i] = f.cond(v0 + i) ? 1 : 0;
     }
     __syncthreads();
-    const uint32_t nb = (ne + kSegBlock - 1) / kSegBlock;
+    const uint32_t nb = MERGE ? part.y : (ne + kSegBlock - 1) / kSegBlock;
     const uint32_t nbw = (uint32_t)warp < nb ? (nb - (uint32_t)warp + kCooWarps - 1) / kCooWarps : 0;
     auto blk_len = [&](uint32_t j) { return min((uint32_t)kSegBlock, ne - j * kSegBlock); };
     auto issue = [&](uint32_t i, int st) {
@@ -647,8 +665,106 @@ __device__ __forceinline__ void pull_coo_w_run(const PullParams& p, const F& f) 
     if constexpr (PF) {
       if (nbw > 0) pload(0);
     }
+    // One 256-edge block of a merging kernel.  What bounds the pull on graphs
+    // whose sources stay in L2 is the instruction issue, so the block is
+    // straight-line code: the edges are sorted by destination, a lane keeps one
+    // running value and passes it on where the next edge has another
+    // destination (predicated, no divergent loop), and the lanes' last runs
+    // are merged by a segmented scan, which a block whose lanes all end on
+    // different destinations skips.  FULL: every slot holds an edge (all blocks
+    // of a tile but its last), so nothing is tested per slot.
+    auto merge_block = [&](auto full, uint32_t j) {
+      constexpr bool FULL = decltype(full)::value;
+      constexpr bool kAllValid = FULL && ALL && F::kCondTrue;
+      const bool in = FULL || (uint32_t)lane * 8 < min((uint32_t)kSegBlock, ne - j * kSegBlock);
+      uint32_t sv[8], wv[8], dv[8];
+      if (in) {
+        const size_t b0 = (size_t)e0 + (size_t)j * kSegBlock + (size_t)lane * 8;
+        const uint4 a = ld16(p.src + b0);
+        const uint4 c = ld16(p.src + b0 + 4);
+        const uint4 q = ld16(p.dloc + b0);
+        sv[0] = a.x; sv[1] = a.y; sv[2] = a.z; sv[3] = a.w;
+        sv[4] = c.x; sv[5] = c.y; sv[6] = c.z; sv[7] = c.w;
+        dv[0] = q.x & 0xffff; dv[1] = q.x >> 16; dv[2] = q.y & 0xffff; dv[3] = q.y >> 16;
+        dv[4] = q.z & 0xffff; dv[5] = q.z >> 16; dv[6] = q.w & 0xffff; dv[7] = q.w >> 16;
+        if (HW) {
+          const uint4 u = ld16(p.wts + b0);
+          const uint4 v = ld16(p.wts + b0 + 4);
+          wv[0] = u.x; wv[1] = u.y; wv[2] = u.z; wv[3] = u.w;
+          wv[4] = v.x; wv[5] = v.y; wv[6] = v.z; wv[7] = v.w;
+        }
+      } else {
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          sv[k] = kPad;
+          dv[k] = 0;
+          wv[k] = 0;
+        }
+      }
+      if (!HW) {
+#pragma unroll
+        for (int k = 0; k < 8; ++k) wv[k] = 1u;
+      }
+      bool vld[8];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) vld[k] = (FULL || sv[k] != kPad) && (F::kCondTrue || s_cond[dv[k]]);
+      if (!ALL) {
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+          if (vld[k]) vld[k] = test_bit(p.fr_bits, sv[k]);
+      }
+      V val[8];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        val[k] = F::identity();
+        if (kAllValid || vld[k]) val[k] = gather(sv[k], wv[k]);
+        // positive functors mark sources outside the frontier with a negative value
+        if (F::kPositive && val[k] < F::identity()) val[k] = F::identity();
+      }
+      // a run reaches the accumulators if one of its edges counts: always, by
+      // its flag where a touched mark is kept, else by a non-identity value
+      auto flush = [&](uint32_t l, V v, bool any) {
+        if (kAllValid && !F::kPositive ? true : kTouch ? any : v != F::identity()) {
+          F::atomic_combine(&s_acc[l], v);
+          if (kTouch) s_touch[l] = 1;
+        }
+      };
+      V acc = val[0];
+      bool any = vld[0];
+#pragma unroll
+      for (int k = 0; k < 7; ++k) {
+        const bool end = dv[k] != dv[k + 1];
+        if (end) flush(dv[k], acc, any);
+        acc = end ? val[k + 1] : F::combine(acc, val[k + 1]);
+        any = vld[k + 1] || (any && !end);
+      }
+      // last runs: equal destinations sit in consecutive lanes; a segmented
+      // scan leaves each segment's total in its last lane
+      const uint32_t prev = __shfl_up_sync(0xffffffffu, dv[7], 1);
+      const uint32_t heads = __ballot_sync(0xffffffffu, lane == 0 || dv[7] != prev);
+      if (heads != 0xffffffffu) {
+        const int s0 = 31 - __clz(heads & (0xffffffffu >> (31 - lane)));
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+          const V t = __shfl_up_sync(0xffffffffu, acc, d);
+          if (lane - d >= s0) acc = F::combine(t, acc);
+        }
+        if (kTouch && !kAllValid) {
+          const uint32_t seg = (0xffffffffu >> (31 - lane)) & (0xffffffffu << s0);
+          any = (__ballot_sync(0xffffffffu, any) & seg) != 0;
+        }
+      }
+      if (lane == 31 || ((heads >> (lane + 1)) & 1u)) flush(dv[7], acc, any);
+    };
     for (uint32_t i = 0; i < nbw; ++i) {
-      const uint32_t j = (uint32_t)warp + i * kCooWarps;
+      const uint32_t j = part.x + (uint32_t)warp + i * kCooWarps;
+      if constexpr (MERGE) {
+        if ((j + 1) * kSegBlock < ne)
+          merge_block(std::true_type{}, j);
+        else
+          merge_block(std::false_type{}, j);
+        continue;
+      }
       const uint32_t nel = blk_len(j);
       const bool in = (uint32_t)lane * 8 < nel;  // 8-slot groups are wholly in or out
       uint32_t sv[8], wv[8];
@@ -762,51 +878,6 @@ __device__ __forceinline__ void pull_coo_w_run(const PullParams& p, const F& f) 
         F::atomic_combine(&s_acc[l], v);
         if (kTouch) s_touch[l] = 1;
       };
-      if constexpr (MERGE) {
-        // The block is sorted by destination, so a lane's middle runs are
-        // complete and go straight to shared memory, while its first run
-        // (held back when the lane has two or more) and its last run may
-        // continue in the neighbouring lanes.
-        int cur = -1, hd = -1;
-        V acc = F::identity(), ha = F::identity();
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-          if (!vld[k]) continue;
-          const int l = (int)dv[k];
-          if (l != cur) {
-            if (cur >= 0) {
-              if (hd < 0) {
-                hd = cur;
-                ha = acc;
-              } else {
-                flush(cur, acc);
-              }
-            }
-            cur = l;
-            acc = val[k];
-          } else {
-            acc = F::combine(acc, val[k]);
-          }
-        }
-        // a held-back first run joins the previous lane's last run
-        const int nhd = __shfl_down_sync(0xffffffffu, hd, 1);
-        const V nha = __shfl_down_sync(0xffffffffu, ha, 1);
-        const int ptl = __shfl_up_sync(0xffffffffu, cur, 1);
-        if (lane < 31 && nhd >= 0 && nhd == cur) acc = F::combine(acc, nha);
-        if (hd >= 0 && !(lane > 0 && ptl == hd)) flush(hd, ha);
-        // last runs: equal destinations sit in consecutive lanes; a segmented
-        // reduction leaves each segment's total in its last lane
-        const uint32_t heads = __ballot_sync(0xffffffffu, lane == 0 || cur != ptl);
-        const int s0 = 31 - __clz(heads & (0xffffffffu >> (31 - lane)));
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-          const V t = __shfl_up_sync(0xffffffffu, acc, d);
-          if (lane - d >= s0) acc = F::combine(t, acc);
-        }
-        const bool seg_end = lane == 31 || ((heads >> (lane + 1)) & 1u);
-        if (seg_end && cur >= 0) flush(cur, acc);
-        continue;
-      }
       int cur = -1;
       V acc = F::identity();
 #pragma unroll
@@ -837,9 +908,73 @@ __device__ __forceinline__ void pull_coo_w_run(const PullParams& p, const F& f) 
     }
     __syncthreads();
     if (s_fail) break;
+    if constexpr (MERGE) {
+      if (part.z > 1) {  // the tile's other items hold the rest of its edges
+        uint32_t* slab = p.slab + part.w;  // arrivals, 3 unused, nv sums, touched bits
+        uint32_t* sums = slab + 4;
+        uint32_t* tbits = sums + ((nv + 3) & ~3u);
+        for (uint32_t i = (uint32_t)warp * 32u; i < nv; i += kCooThreads) {
+          const uint32_t l = i + (uint32_t)lane;
+          if (l < nv && s_acc[l] != F::identity()) F::slab_combine(sums + l, s_acc[l]);
+          if constexpr (kTouch) {
+            const uint32_t word = __ballot_sync(0xffffffffu, l < nv && s_touch[l] != 0);
+            if (lane == 0 && word) atomicOr(tbits + (i >> 5), word);
+          }
+        }
+        __threadfence();
+        __syncthreads();
+        if (tid == 0) {
+          s_last = atomicAdd(slab, 1u) == part.z - 1;
+          if (s_last) *slab = 0;
+        }
+        __syncthreads();
+        if (!s_last) continue;
+        __threadfence();
+        for (uint32_t i0 = (uint32_t)warp * 32u; i0 < nv; i0 += 4 * kCooThreads) {
+          uint32_t raw[4], word[4];
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            const uint32_t i = i0 + (uint32_t)u * kCooThreads, l = i + (uint32_t)lane;
+            raw[u] = l < nv ? __ldcg(sums + l) : 0u;
+            if constexpr (kTouch) word[u] = i < nv ? __ldcg(tbits + (i >> 5)) : 0u;
+          }
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            const uint32_t i = i0 + (uint32_t)u * kCooThreads, l = i + (uint32_t)lane;
+            if (l < nv) {
+              s_acc[l] = F::slab_decode(raw[u]);
+              if (raw[u]) sums[l] = 0;
+            }
+            if constexpr (kTouch) {
+              if (l < nv) s_touch[l] = (word[u] >> lane) & 1u;
+              __syncwarp();
+              if (lane == 0 && word[u]) tbits[i >> 5] = 0;
+            }
+          }
+        }
+        __syncthreads();
+      }
+    }
+    // The commits go kCommitAhead destinations per thread at a time, every
+    // load (degree bounds, what the functor's commit reads) issued before the
+    // first store.
+    constexpr int kCommitAhead = 4;
     if constexpr (NOOUT) {
-      for (uint32_t l = tid; l < nv; l += kCooThreads)
-        if (s_acc[l] != F::identity() && (F::kCondTrue || s_cond[l])) f.commit(v0 + l, s_acc[l]);
+      for (uint32_t l0 = tid; l0 < nv; l0 += kCommitAhead * kCooThreads) {
+        CommitIn x[kCommitAhead];
+        bool on[kCommitAhead];
+#pragma unroll
+        for (int u = 0; u < kCommitAhead; ++u) {
+          const uint32_t l = l0 + u * kCooThreads;
+          on[u] = l < nv && s_acc[l] != F::identity() && (F::kCondTrue || s_cond[l]);
+          if (on[u]) x[u] = f.commit_load(v0 + l);
+        }
+#pragma unroll
+        for (int u = 0; u < kCommitAhead; ++u) {
+          const uint32_t l = l0 + u * kCooThreads;
+          if (on[u]) f.commit_apply(v0 + l, x[u], s_acc[l]);
+        }
+      }
       __syncthreads();
       continue;
     }
@@ -848,7 +983,6 @@ __device__ __forceinline__ void pull_coo_w_run(const PullParams& p, const F& f) 
       // the vertex step of kCommitAhead 32-vertex groups per round: every
       // group's loads (degree bounds, rank, previous rank, frontier word)
       // are issued before the first group's arithmetic and stores
-      constexpr int kCommitAhead = 4;
       for (uint32_t b0 = base0 + (uint32_t)warp * 32u; b0 < v0 + nv; b0 += kCommitAhead * kCooThreads) {
         typename F::FinishIn x[kCommitAhead];
         uint32_t dg[kCommitAhead];
@@ -886,30 +1020,54 @@ __device__ __forceinline__ void pull_coo_w_run(const PullParams& p, const F& f) 
       __syncthreads();
       continue;
     }
-    for (uint32_t bb = base0 + (uint32_t)warp * 32u; bb < v0 + nv; bb += kCooThreads) {
-      const uint32_t v = bb + (uint32_t)lane;
-      bool act = false;
-      uint32_t dg = 0;
-      if (v >= v0 && v < v0 + nv) {
-        const uint32_t l = v - v0;
-        const bool touched = F::kPositive ? (s_acc[l] != F::identity()) : (s_touch[l] != 0);
-        if constexpr (kFin) {
-          dg = __ldg(p.deg_off + v + 1) - __ldg(p.deg_off + v);
-          my_l1 += f.finish(v, touched, s_acc[l], dg);
-          act = touched;
-        } else if (touched && (F::kCondTrue || s_cond[l])) {
-          act = f.commit(v, s_acc[l]);
+    if constexpr (!kFin) {
+      for (uint32_t b0 = base0 + (uint32_t)warp * 32u; b0 < v0 + nv; b0 += kCommitAhead * kCooThreads) {
+        CommitIn x[kCommitAhead];
+        uint32_t dg[kCommitAhead];
+        bool on[kCommitAhead];
+#pragma unroll
+        for (int u = 0; u < kCommitAhead; ++u) {
+          const uint32_t v = b0 + (uint32_t)u * kCooThreads + (uint32_t)lane, l = v - v0;
+          on[u] = v >= v0 && v < v0 + nv && (F::kPositive ? (s_acc[l] != F::identity()) : (s_touch[l] != 0)) &&
+                  (F::kCondTrue || s_cond[l]);
+          dg[u] = 0;
+          if (on[u]) {
+            dg[u] = __ldg(p.deg_off + v + 1) - __ldg(p.deg_off + v);
+            x[u] = f.commit_load(v);
+          }
+        }
+#pragma unroll
+        for (int u = 0; u < kCommitAhead; ++u) {
+          const uint32_t bb = b0 + (uint32_t)u * kCooThreads;
+          if (bb >= v0 + nv) break;  // warp-uniform
+          const uint32_t v = bb + (uint32_t)lane;
+          bool act = false;
+          if (on[u]) act = f.commit_apply(v, x[u], s_acc[v - v0]);
+          const uint32_t word = __ballot_sync(0xffffffffu, act);
+          if (act) my_deg += dg[u];
+          if (lane == 0 && word) {
+            atomicOr(p.next_bits + (bb >> 5), word);
+            my_cnt += __popc(word);
+          }
         }
       }
-      const uint32_t word = __ballot_sync(0xffffffffu, act);
-      if (kFin) {
+    } else {
+      for (uint32_t bb = base0 + (uint32_t)warp * 32u; bb < v0 + nv; bb += kCooThreads) {
+        const uint32_t v = bb + (uint32_t)lane;
+        bool act = false;
+        uint32_t dg = 0;
+        if (v >= v0 && v < v0 + nv) {
+          const uint32_t l = v - v0;
+          act = s_acc[l] != F::identity();
+          dg = __ldg(p.deg_off + v + 1) - __ldg(p.deg_off + v);
+          my_l1 += f.finish(v, act, s_acc[l], dg);
+        }
+        const uint32_t word = __ballot_sync(0xffffffffu, act);
         if (act) my_deg += dg;
-      } else if (act) {
-        my_deg += __ldg(p.deg_off + v + 1) - __ldg(p.deg_off + v);
-      }
-      if (lane == 0 && word) {
-        atomicOr(p.next_bits + (bb >> 5), word);
-        my_cnt += __popc(word);
+        if (lane == 0 && word) {
+          atomicOr(p.next_bits + (bb >> 5), word);
+          my_cnt += __popc(word);
+        }
       }
     }
     __syncthreads();

@@ -18,6 +18,9 @@ struct MinI32 {
   __device__ static value_t identity() { return 0x7fffffff; }
   __device__ static value_t combine(value_t a, value_t b) { return a < b ? a : b; }
   __device__ static void atomic_combine(value_t* s, value_t v) { atomicMin(s, v); }
+  // a COO tile's slab word (0 = identity): the distance below INT_MAX
+  __device__ static void slab_combine(uint32_t* s, value_t v) { atomicMax(s, 0x7fffffffu - (uint32_t)v); }
+  __device__ static value_t slab_decode(uint32_t r) { return (value_t)(0x7fffffffu - r); }
 };
 struct MinU32 {
   using value_t = uint32_t;
@@ -27,6 +30,8 @@ struct MinU32 {
   __device__ static value_t identity() { return 0xffffffffu; }
   __device__ static value_t combine(value_t a, value_t b) { return a < b ? a : b; }
   __device__ static void atomic_combine(value_t* s, value_t v) { atomicMin(s, v); }
+  __device__ static void slab_combine(uint32_t* s, value_t v) { atomicMax(s, ~v); }
+  __device__ static value_t slab_decode(uint32_t r) { return ~r; }
 };
 struct SumF32 {
   using value_t = float;
@@ -36,6 +41,8 @@ struct SumF32 {
   __device__ static value_t identity() { return 0.0f; }
   __device__ static value_t combine(value_t a, value_t b) { return a + b; }
   __device__ static void atomic_combine(value_t* s, value_t v) { atomicAdd(s, v); }
+  __device__ static void slab_combine(uint32_t* s, value_t v) { atomicAdd(reinterpret_cast<float*>(s), v); }
+  __device__ static value_t slab_decode(uint32_t r) { return __uint_as_float(r); }
 };
 
 // BFS_F, app/BFS.C:26-75.  cond = unvisited; update = first writer becomes
@@ -52,11 +59,13 @@ struct BfsF : MinU32 {
   int32_t round;
   __device__ bool cond(uint32_t d) const { return __ldcg(parents + d) == -1; }
   __device__ value_t gather(uint32_t s, uint32_t) const { return s; }
-  __device__ bool commit(uint32_t d, value_t acc) const {
+  __device__ CommitIn commit_load(uint32_t) const { return CommitIn{}; }
+  __device__ bool commit_apply(uint32_t d, CommitIn, value_t acc) const {
     parents[d] = (int32_t)acc;
     if (levels) levels[d] = round;
     return true;
   }
+  __device__ bool commit(uint32_t d, value_t acc) const { return commit_apply(d, commit_load(d), acc); }
   __device__ bool update_atomic(uint32_t s, uint32_t d, uint32_t) const {
     if (atomicCAS(parents + d, -1, (int32_t)s) == -1) {
       if (levels) levels[d] = round;
@@ -78,14 +87,16 @@ struct CcF : MinI32 {
   int32_t* prev;
   __device__ bool cond(uint32_t) const { return true; }
   __device__ value_t gather(uint32_t s, uint32_t) const { return __ldg(prev + s); }
-  __device__ bool commit(uint32_t d, value_t acc) const {
-    const int32_t orig = ids[d];
+  __device__ CommitIn commit_load(uint32_t d) const { return CommitIn{(uint32_t)ids[d], (uint32_t)prev[d]}; }
+  __device__ bool commit_apply(uint32_t d, CommitIn in, value_t acc) const {
+    const int32_t orig = (int32_t)in.a;
     if (acc < orig) {
       ids[d] = acc;
-      return orig == prev[d];
+      return orig == (int32_t)in.b;
     }
     return false;
   }
+  __device__ bool commit(uint32_t d, value_t acc) const { return commit_apply(d, commit_load(d), acc); }
   __device__ bool update_atomic(uint32_t s, uint32_t d, uint32_t) const {
     const int32_t v = __ldcg(ids + s);
     const int32_t old = atomicMin(ids + d, v);
@@ -115,10 +126,12 @@ struct PrT : SumF32 {
   __device__ value_t gather_pol(uint32_t s, uint32_t, uint64_t pol) const {
     return gg::ld_keep_f32(contrib + s, pol);
   }
-  __device__ bool commit(uint32_t d, value_t acc) const {
-    acc_out[d] += acc;
+  __device__ CommitIn commit_load(uint32_t d) const { return CommitIn{__float_as_uint(acc_out[d]), 0u}; }
+  __device__ bool commit_apply(uint32_t d, CommitIn in, value_t acc) const {
+    acc_out[d] = __uint_as_float(in.a) + acc;
     return true;
   }
+  __device__ bool commit(uint32_t d, value_t acc) const { return commit_apply(d, commit_load(d), acc); }
   __device__ bool update_atomic(uint32_t s, uint32_t d, uint32_t) const {
     atomicAdd(acc_out + d, __ldg(contrib + s));
     return true;
@@ -196,10 +209,15 @@ struct SpmvF : SumF32 {
   __device__ value_t gather_pol(uint32_t s, uint32_t w, uint64_t pol) const {
     return gg::ld_keep_f32(x + s, pol) * wv(w);
   }
-  __device__ bool commit(uint32_t d, value_t acc) const {
-    y[yi(d)] += acc;
+  __device__ CommitIn commit_load(uint32_t d) const {
+    const uint32_t i = yi(d);
+    return CommitIn{__float_as_uint(y[i]), i};
+  }
+  __device__ bool commit_apply(uint32_t, CommitIn in, value_t acc) const {
+    y[in.b] = __uint_as_float(in.a) + acc;
     return true;
   }
+  __device__ bool commit(uint32_t d, value_t acc) const { return commit_apply(d, commit_load(d), acc); }
   __device__ bool update_atomic(uint32_t s, uint32_t d, uint32_t w) const {
     atomicAdd(y + yi(d), __ldg(x + s) * wv(w));
     return true;
@@ -218,16 +236,18 @@ struct BfF : MinI32 {
   int32_t* visited;
   __device__ bool cond(uint32_t) const { return true; }
   __device__ value_t gather(uint32_t s, uint32_t w) const { return __ldcg(sp + s) + (int32_t)w; }
-  __device__ bool commit(uint32_t d, value_t acc) const {
-    if (acc < sp[d]) {
+  __device__ CommitIn commit_load(uint32_t d) const { return CommitIn{(uint32_t)sp[d], (uint32_t)visited[d]}; }
+  __device__ bool commit_apply(uint32_t d, CommitIn in, value_t acc) const {
+    if (acc < (int32_t)in.a) {
       sp[d] = acc;
-      if (visited[d] == 0) {
+      if (in.b == 0) {
         visited[d] = 1;
         return true;
       }
     }
     return false;
   }
+  __device__ bool commit(uint32_t d, value_t acc) const { return commit_apply(d, commit_load(d), acc); }
   __device__ bool update_atomic(uint32_t s, uint32_t d, uint32_t w) const {
     const int32_t nd = __ldcg(sp + s) + (int32_t)w;
     const int32_t old = atomicMin(sp + d, nd);
@@ -247,11 +267,13 @@ struct BcF : SumF32 {
   const uint8_t* visited;
   __device__ bool cond(uint32_t d) const { return visited[d] == 0; }
   __device__ value_t gather(uint32_t s, uint32_t) const { return __ldcg(values + s); }
-  __device__ bool commit(uint32_t d, value_t acc) const {
-    const float old = values[d];
+  __device__ CommitIn commit_load(uint32_t d) const { return CommitIn{__float_as_uint(values[d]), 0u}; }
+  __device__ bool commit_apply(uint32_t d, CommitIn in, value_t acc) const {
+    const float old = __uint_as_float(in.a);
     values[d] = old + acc;
     return old == 0.0f;
   }
+  __device__ bool commit(uint32_t d, value_t acc) const { return commit_apply(d, commit_load(d), acc); }
   __device__ bool update_atomic(uint32_t s, uint32_t d, uint32_t) const {
     return atomicAdd(values + d, __ldcg(values + s)) == 0.0f;
   }

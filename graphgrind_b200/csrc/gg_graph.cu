@@ -367,6 +367,53 @@ int build_bu_index(gg_graph_s* g) {
   return GG_OK;
 }
 
+// Work items of the merging COO pulls (pull_coo_w_run).  An item aims at half
+// the edges a resident CTA takes on average (4 CTAs per SM), so that the last
+// CTAs finish together, but at no fewer than four edges per destination of the
+// tile: below that the passes over the tile's accumulators and its slab cost
+// more than the balance gains (PageRank pull, R-MAT-20 / R-MAT-22 with
+// 2^18-edge tiles: half an average share and 4 edges per destination 87.7 /
+// 218 us, a quarter and 2 edges 93.6 / 216 us, whole tiles 92 / 365 us).  A
+// tile of less than one and a half items stays whole.
+static int build_coo_items(gg_graph_s* g) {
+  const uint64_t per_cta = g->coo_len / ((uint64_t)g->num_sms * 4);
+  std::vector<uint4> items;
+  uint64_t slab = 0;
+  struct Part {
+    uint32_t tile, first, blocks, parts;
+    uint64_t slab;
+  };
+  std::vector<Part> parts;
+  for (uint32_t t = 0; t < g->coo_tiles.count; ++t) {
+    const uint4 td = g->coo_tiles.host[t];
+    const uint32_t nb = (td.w + kSegBlock - 1) / kSegBlock;
+    const uint64_t want = std::max<uint64_t>({per_cta / 2, 4ull * td.y, kCooItemMinEdges});
+    const uint32_t k = (uint32_t)std::min<uint64_t>(nb, std::max<uint64_t>(1, (td.w + want / 2) / want));
+    uint32_t b = 0;
+    for (uint32_t i = 0; i < k; ++i) {
+      const uint32_t e = (uint32_t)((uint64_t)nb * (i + 1) / k);
+      parts.push_back(Part{t, b, e - b, k, slab});
+      b = e;
+    }
+    if (k > 1) slab += 4 + ((td.y + 3) & ~3u) + ((td.y + 127) / 128) * 4;
+  }
+  if (slab >= (1ull << 32)) return fail(GG_ERR_SIZE, "COO slabs exceed 2^32 words");
+  std::stable_sort(parts.begin(), parts.end(), [](const Part& a, const Part& b) { return a.blocks > b.blocks; });
+  for (const Part& q : parts) {
+    items.push_back(g->coo_tiles.host[q.tile]);
+    items.push_back(make_uint4(q.first, q.blocks, q.parts, (uint32_t)q.slab));
+  }
+  g->coo_item_count = (uint32_t)parts.size();
+  GG_TRY(dev_alloc(g, &g->d_coo_items, std::max<size_t>(items.size(), 1)));
+  if (!items.empty())
+    GG_CUDA(cudaMemcpy(g->d_coo_items, items.data(), sizeof(uint4) * items.size(), cudaMemcpyHostToDevice));
+  if (slab) {
+    GG_TRY(dev_alloc(g, &g->d_coo_slab, slab));
+    GG_CUDA(cudaMemset(g->d_coo_slab, 0, 4 * slab));
+  }
+  return GG_OK;
+}
+
 static int build_coo(gg_graph_s* g, const uint32_t* h_in_off) {
   const uint32_t n = g->n;
   const uint64_t m = g->m;
@@ -505,6 +552,7 @@ static int build_coo(gg_graph_s* g, const uint32_t* h_in_off) {
   for (size_t t = 0; t < segs.size(); ++t)
     tiles[t] = make_uint4(segs[t].x, segs[t].y, pad_start[t], (segs[t].w + 7u) & ~7u);
   GG_TRY(upload_tiles(g, g->coo_tiles, tiles));
+  GG_TRY(build_coo_items(g));
   // destination ranges that no tile covers (no in-edges at all): a vertex
   // step run at the tiles' commits visits them separately
   std::vector<uint2> gaps;
@@ -657,6 +705,8 @@ static void graph_release(gg_graph_s* g) {
     cudaFree(s.d_rows);
   }
   cudaFree(g->coo_tiles.d_tiles);
+  cudaFree(g->d_coo_items);
+  cudaFree(g->d_coo_slab);
   cudaFree(g->d_coo_gaps);
   cudaFree(g->d_coo_src);
   cudaFree(g->d_coo_dloc);

@@ -282,6 +282,9 @@ int pull_launch(gg_graph_s* g, gg_frontier_s* in, gg_frontier_s* out, const F& f
     p.dloc = g->d_coo_dloc;
     p.wts = g->d_coo_w;
     p.off = nullptr;
+    p.items = g->d_coo_items;
+    p.nitems = g->coo_item_count;
+    p.slab = g->d_coo_slab;
   } else {
     p.tiles = g->csc_tiles[orient].d_tiles;
     p.ntiles = g->csc_tiles[orient].count;
@@ -329,6 +332,7 @@ int pull_launch(gg_graph_s* g, gg_frontier_s* in, gg_frontier_s* out, const F& f
     static DeviceOnce opted_mg[2];
     constexpr int kFlags = coo_w_flag_bytes<F, false>(), kFlagsNoOut = coo_w_flag_bytes<F, true>();
     auto launch_w = [&](auto kern, int stages, DeviceOnce& once, int flags) -> int {
+      const uint32_t work = g->coo_kernel >= 6 ? p.nitems : p.ntiles;  // the merging kernels (6, 7) take items
       const size_t smem = coo_w_smem_bytes(kHW, stages, 4, p.tv, flags);
       const int ok = once.get(g->device, [&]() {
         return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -340,7 +344,7 @@ int pull_launch(gg_graph_s* g, gg_frontier_s* in, gg_frontier_s* out, const F& f
       int blocks = 1;
       GG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, kern, kCooThreads, smem));
       if (blocks < 1) blocks = 1;
-      const int grid = (int)std::min<uint64_t>((uint64_t)g->num_sms * blocks, p.ntiles);
+      const int grid = (int)std::min<uint64_t>((uint64_t)g->num_sms * blocks, work);
       kern<<<grid, kCooThreads, smem, g->stream>>>(p, f);
       GG_CUDA(cudaGetLastError());
       g->kernels++;
