@@ -187,36 +187,38 @@ static int to_host(gg_graph_s* g, T* host, const T* dev, uint64_t n) {
 static int run_bfs(gg_graph_s* g, uint32_t start, int32_t* parents, int32_t* levels, gg_run_stats* st) {
   const uint32_t n = g->n;
   g->kernels = 0;
-  DevBuf<int32_t> par, lev;
+  DevBuf<int32_t> parb, levb;
+  DevBuf<uint32_t> arena;
+  int32_t *par = nullptr, *lev = nullptr;
   // every level in one cooperative launch (its dense levels pull over the CSC;
   // a graph told to pull over the COO keeps the host loop for them), which
   // writes levels only when they are asked for
   const bool full = g->device_loop == 2 && !g->transposed && g->dense_policy != 2;
-  const bool want_lev = levels || !full;
-  GG_TRY(par.alloc(g, n));
-  if (want_lev) GG_TRY(lev.alloc(g, n));
   EventTimer tm(g->stream);
-  GG_TRY(fill<int32_t>(g, par.p, n, -1));
-  GG_TRY(set_one<int32_t>(g, par.p, start, (int32_t)start));
-  if (want_lev) {
-    GG_TRY(fill<int32_t>(g, lev.p, n, -1));
-    GG_TRY(set_one<int32_t>(g, lev.p, start, 0));
-  }
   FrontierHold F;
   int32_t round = 0;
   uint64_t trav = 0;
   const int64_t thr = app_threshold(g);
-  if (full)
-    GG_TRY(bfs_device_full(g, start, par.p, lev.p, (uint64_t)thr));
-  else
+  if (full) {
+    GG_TRY(bfs_device_full(g, start, levels != nullptr, arena, &par, &lev, (uint64_t)thr));
+  } else {
+    GG_TRY(parb.alloc(g, n));
+    GG_TRY(levb.alloc(g, n));
+    par = parb.p;
+    lev = levb.p;
+    GG_TRY(fill<int32_t>(g, par, n, -1));
+    GG_TRY(set_one<int32_t>(g, par, start, (int32_t)start));
+    GG_TRY(fill<int32_t>(g, lev, n, -1));
+    GG_TRY(set_one<int32_t>(g, lev, start, 0));
     GG_TRY(gg_frontier_single(g, start, &F.f));
+  }
   while (F.f && F.f->dm > 0) {
     if (g->device_loop && (int64_t)(F.f->dm + F.f->out_edges) <= thr && F.f->out_edges > 0) {
       // sparse levels run on the device until the frontier empties or turns dense
       int32_t levels_run = 0;
       uint64_t t = 0;
       gg_frontier_s* cur = F.release();
-      const int rc = bfs_device_levels(g, &cur, par.p, lev.p, round + 1, (uint64_t)thr, &levels_run, &t);
+      const int rc = bfs_device_levels(g, &cur, par, lev, round + 1, (uint64_t)thr, &levels_run, &t);
       F.f = cur;
       if (rc) return rc;
       round += levels_run;
@@ -225,34 +227,38 @@ static int run_bfs(gg_graph_s* g, uint32_t start, int32_t* parents, int32_t* lev
     }
     ++round;
     BfsF f;
-    f.parents = par.p;
-    f.levels = lev.p;
+    f.parents = par;
+    f.levels = lev;
     f.round = round;
     trav += F.f->out_edges;
     gg_frontier_s* out = nullptr;
     GG_TRY(edge_map(g, F.f, f, thr, 0, &out));
     F.reset(out);
   }
-  const int32_t* par_out = par.p;
-  const int32_t* lev_out = lev.p;
+  const int32_t* par_out = par;
+  const int32_t* lev_out = lev;
   const int pslot = g->async_results && g->ws.d_order[2] ? 2 : 0;  // the given-order array of the parents
   if (g->relabeled && parents) {
     int32_t* tp = reinterpret_cast<int32_t*>(g->ws.d_order[pslot]);
     GG_TRY(slot_write_wait(g, pslot));
     k_ids_to_given<<<generic_grid(g, n), kGenericThreads, 0, g->stream>>>(n, g->d_new_of_old, g->d_old_of_new,
-                                                                          par.p, tp);
+                                                                          par, tp);
     g->kernels++;
     par_out = tp;
   }
-  if (parents && !g->relabeled) GG_TRY(given_order<int32_t>(g, par.p, pslot, &par_out));
-  if (levels) GG_TRY(given_order<int32_t>(g, lev.p, 1, &lev_out));
-  const double ms = tm.stop();
-  // the all-levels launch is read back after the device work it feeds was
-  // queued behind it, so that the stream does not idle for the host
-  if (full) GG_TRY(bfs_device_full_result(g, &round, &trav));
+  if (parents && !g->relabeled) GG_TRY(given_order<int32_t>(g, par, pslot, &par_out));
+  if (levels) GG_TRY(given_order<int32_t>(g, lev, 1, &lev_out));
+  tm.mark();
+  // the all-levels launch is read back after the device work it feeds and the
+  // copies of its results were queued behind it: one wait for all of them
+  if (full) GG_TRY(bfs_device_full_begin_result(g));
   GG_TRY(to_host(g, parents, par_out, n));
   GG_TRY(to_host(g, levels, lev_out, n));
-  fill_stats(st, ms, round, trav, g->kernels);
+  if (full) {
+    GG_CUDA(cudaStreamSynchronize(g->stream));
+    GG_TRY(bfs_device_full_result(g, &round, &trav));
+  }
+  fill_stats(st, tm.elapsed(), round, trav, g->kernels);
   return GG_OK;
 }
 

@@ -166,7 +166,7 @@ struct gg_graph_s {
   int sparse_div = 20;  // the apps' edgeMap threshold is m / sparse_div (app/*.C pass m/20)
   int device_loop = 2;  // 2: the whole BFS in one cooperative launch; 1: runs of sparse levels; 0: none
   int cc_algo = 0;      // Components on symmetric graphs: 0 label propagation, 1 union-find
-  int loop_ctas_per_sm = 0;  // CTAs per SM of the device BFS loops (capped by occupancy); 0: 4 / 8 by loop
+  int loop_ctas_per_sm = 0;  // CTAs per SM of the device BFS loops (capped by occupancy); 0: 2 / 4 by loop
   uint32_t loop_wait_budget = 1u << 22;  // spins of the BFS level loop's grid-barrier wait
   int early_kernel = 3;  // early-exit dense pull: 0 one lane per destination, 1 8-lane groups, 2 one lane per
                          // destination reading 4 in-edges per load, 3 the same over in-lists with hub sources

@@ -6,14 +6,24 @@
 // reads the next frontier's size and out-degree and applies edgeMap's
 // direction rule (size + out-degree > threshold means a dense level): the
 // launch returns when the frontier is empty, needs a dense level, or a level
-// cap is reached, and the host continues with edgeMap.  Each level's queue
-// chunks of 256 frontier vertices are spread over the CTAs; inside a CTA a
-// block prefix sum over the chunk's degrees balances its edges over the
-// threads.  The barrier wait is bounded: on expiry the kernel records an error
+// cap is reached, and the host continues with edgeMap.  A level's
+// edges go to the CTAs in windows of 512: every queue slot carries its first
+// edge's offset, and whoever appends a slot notes it as the first of each
+// window whose first edge it holds, so a CTA reaches its window's slots with
+// one load.  The barrier wait is bounded: on expiry the kernel records an error
 // and returns.
 #include "gg_runtime.cuh"
 
 namespace gg {
+
+// Threads of a loop CTA, and edges of a window of a sparse level.  A sparse
+// level of a high-diameter graph costs its latency: the grid barrier (whose
+// arrivals all go to one L2 word) and one window's chain of dependent loads.
+// Wider CTAs make fewer arrivals and hold more of the frontier per window, but
+// a window's block barriers cost more (2049^2 grid, 125 levels: gg_bfs 1.85 /
+// 1.59 / 2.16 ms with 256 / 512 / 1024 threads; R-MAT-22 0.53 / 0.52 / 0.53).
+constexpr int kLoopThreads = 512;
+constexpr int kLoopWarps = kLoopThreads / 32;
 
 // One frontier's counters; the loops keep three, by level mod 3.
 struct LoopSlot {
@@ -92,15 +102,22 @@ __device__ __forceinline__ bool grid_barrier(unsigned* bar, unsigned target, uns
   return *s_ok != 0;
 }
 
+// A queue slot whose edges start at eoff notes itself as the first slot of
+// every window whose first edge it holds, so that a CTA finds its window's
+// slots with one load.
+__device__ __forceinline__ void note_windows(uint32_t* wst, uint32_t slot, uint32_t eoff, uint32_t deg) {
+  for (uint64_t w = ((uint64_t)eoff + kLoopThreads - 1) / kLoopThreads; w * kLoopThreads < (uint64_t)eoff + deg; ++w)
+    wst[w] = slot;
+}
+
 // Warp-cooperative append to the next frontier (every lane calls it).  A
 // vertex with out-edges gets its queue slot and its first edge offset from one
 // 64-bit atomic (slots in the high half, edges in the low half), so slot order
 // is edge-offset order; a vertex without out-edges goes to the far end.
 __device__ __forceinline__ void loop_append(bool add, uint32_t u, uint32_t deg, uint32_t* nq, uint32_t* neo,
-                                            uint32_t n, unsigned long long* packed, unsigned long long* zeros,
-                                            uint32_t* nbits = nullptr) {
+                                            uint32_t* nwst, uint32_t n, unsigned long long* packed,
+                                            unsigned long long* zeros) {
   const int lane = threadIdx.x & 31;
-  if (nbits && add) atomicOr(nbits + (u >> 5), 1u << (u & 31));
   const uint32_t lanemask_lt = (1u << lane) - 1u;
   const bool pos = add && deg > 0, zer = add && deg == 0;
   uint32_t inc = pos ? deg : 0u;
@@ -120,6 +137,7 @@ __device__ __forceinline__ void loop_append(bool add, uint32_t u, uint32_t deg, 
       const uint64_t slot = (old >> 32) + __popc(bal & lanemask_lt);
       nq[slot] = u;
       neo[slot] = (uint32_t)old + inc - deg;
+      note_windows(nwst, (uint32_t)slot, (uint32_t)old + inc - deg, deg);
     }
   }
   const uint32_t zb = __ballot_sync(0xffffffffu, zer);
@@ -132,138 +150,123 @@ __device__ __forceinline__ void loop_append(bool add, uint32_t u, uint32_t deg, 
   }
 }
 
-// block-wide exclusive scan of two 32-bit counts (blockDim.x == 256)
-__device__ __forceinline__ void block_scan2(uint32_t a, uint32_t b, uint32_t* ea, uint32_t* eb, uint32_t* ta,
-                                           uint32_t* tb, uint32_t (*s)[8]) {
+// block-wide exclusive scan of one 64-bit value (kLoopThreads threads)
+__device__ __forceinline__ unsigned long long block_scan(unsigned long long a, unsigned long long* total,
+                                                         unsigned long long* s) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  uint32_t x = a, y = b;
+  unsigned long long x = a;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t u = __shfl_up_sync(0xffffffffu, x, o), w = __shfl_up_sync(0xffffffffu, y, o);
-    if (lane >= o) {
-      x += u;
-      y += w;
-    }
+    const unsigned long long u = __shfl_up_sync(0xffffffffu, x, o);
+    if (lane >= o) x += u;
   }
-  if (lane == 31) {
-    s[0][warp] = x;
-    s[1][warp] = y;
-  }
+  if (lane == 31) s[warp] = x;
   __syncthreads();
-  uint32_t pa = 0, pb = 0, sa = 0, sb = 0;
-  for (int w = 0; w < 8; ++w) {
-    if (w < warp) {
-      pa += s[0][w];
-      pb += s[1][w];
-    }
-    sa += s[0][w];
-    sb += s[1][w];
+  unsigned long long before = 0, all = 0;
+#pragma unroll
+  for (int w = 0; w < kLoopWarps; ++w) {
+    if (w < warp) before += s[w];
+    all += s[w];
   }
-  *ea = pa + x - a;
-  *eb = pb + y - b;
-  *ta = sa;
-  *tb = sb;
-  __syncthreads();
+  *total = all;
+  return before + x - a;
 }
 
 // Block-wide append to the next frontier (every thread calls it): one
 // 64-bit atomic per CTA for the vertices with out-edges (slots and edge
 // offsets, as loop_append) and one for those without.
 __device__ __forceinline__ void block_append(bool add, uint32_t u, uint32_t deg, uint32_t* nq, uint32_t* neo,
-                                             uint32_t n, unsigned long long* packed, unsigned long long* zeros,
-                                             uint32_t* nbits, uint32_t (*s_scan)[8], unsigned long long* s_base) {
+                                             uint32_t* nwst, uint32_t n, unsigned long long* packed,
+                                             unsigned long long* zeros, uint32_t* nbits,
+                                             unsigned long long* s_scan, unsigned long long* s_base) {
   if (nbits && add) atomicOr(nbits + (u >> 5), 1u << (u & 31));
   const bool pos = add && deg > 0, zer = add && deg == 0;
-  // counts packed as (with out-edges << 16) | without; at most 256 each
-  uint32_t ec, ed, tc, td;
-  block_scan2((pos ? 1u << 16 : 0u) | (zer ? 1u : 0u), pos ? deg : 0u, &ec, &ed, &tc, &td, s_scan);
-  if (threadIdx.x == 0) {
-    s_base[0] = (tc >> 16) ? atomicAdd(packed, ((unsigned long long)(tc >> 16) << 32) | td) : 0ull;
-    s_base[1] = (tc & 0xffffu) ? atomicAdd(zeros, (unsigned long long)(tc & 0xffffu)) : 0ull;
-  }
+  // counts packed as (with out-edges << 48) | (without << 32) | edges; at most kLoopThreads vertices
+  unsigned long long total;
+  const unsigned long long ex = block_scan((pos ? 1ull << 48 : 0ull) | (zer ? 1ull << 32 : 0ull) | (pos ? deg : 0u),
+                                           &total, s_scan);
+  const uint32_t np = (uint32_t)(total >> 48), nz = (uint32_t)(total >> 32) & 0xffffu;
+  if (threadIdx.x == 0 && np) s_base[0] = atomicAdd(packed, ((unsigned long long)np << 32) | (uint32_t)total);
+  if (threadIdx.x == 32 && nz) s_base[1] = atomicAdd(zeros, (unsigned long long)nz);
   __syncthreads();
   if (pos) {
     const unsigned long long old = s_base[0];
-    const uint64_t slot = (old >> 32) + (ec >> 16);
+    const uint32_t slot = (uint32_t)(old >> 32) + (uint32_t)(ex >> 48);
+    const uint32_t eoff = (uint32_t)old + (uint32_t)ex;
     nq[slot] = u;
-    neo[slot] = (uint32_t)old + ed;
+    neo[slot] = eoff;
+    note_windows(nwst, slot, eoff, deg);
   } else if (zer) {
-    nq[n - 1 - (s_base[1] + (ec & 0xffffu))] = u;
+    nq[n - 1 - (s_base[1] + ((uint32_t)(ex >> 32) & 0xffffu))] = u;
   }
 }
 
-// One sparse (top-down) level, this CTA's contiguous share of its E edges:
-// queue q with slot edge offsets eo (k slots, each with >= 1 edge); vertices
-// reached for the first time go to nq/neo (and nbits when given).
+// The shared memory of a sparse level's window.
+struct PushShared {
+  uint32_t eo[kLoopThreads];
+  uint32_t v[kLoopThreads];
+  uint32_t beg[kLoopThreads];
+  unsigned long long scan[kLoopWarps];
+  unsigned long long base[2];
+};
+
+// One sparse (top-down) level, this CTA's windows of its E edges: queue q with
+// slot edge offsets eo (k slots, each with >= 1 edge) and window starts wst;
+// vertices reached for the first time go to nq/neo/nwst (and nbits when given).
+// mark: the value written to `parents` is the level r instead of the parent.
 __device__ __noinline__ void push_level(const uint32_t* __restrict__ off, const uint32_t* __restrict__ idx,
-                                           int32_t* parents, int32_t* levels, const uint32_t* q, const uint32_t* eo,
-                                           uint32_t* nq, uint32_t* neo, uint64_t k, uint64_t E, uint32_t n, int32_t r,
-                                           unsigned long long* packed, unsigned long long* zeros, uint32_t* nbits,
-                                           uint32_t* s_eo, uint32_t* s_v, uint32_t* s_beg, uint32_t (*s_scan)[8],
-                                           unsigned long long* s_base) {
+                                        int32_t* parents, int32_t* levels, const uint32_t* q, const uint32_t* eo,
+                                        const uint32_t* wst, uint32_t* nq, uint32_t* neo, uint32_t* nwst, uint64_t k,
+                                        uint64_t E, uint32_t n, int32_t r, int mark, unsigned long long* packed,
+                                        unsigned long long* zeros, uint32_t* nbits, PushShared* s) {
   const int tid = threadIdx.x;
-  // this CTA's contiguous share of the level's edges
-  const uint64_t per = (E + gridDim.x - 1) / gridDim.x;
-  const uint64_t b0 = (uint64_t)blockIdx.x * per, b1 = b0 + per < E ? b0 + per : E;
-  if (b0 < b1) {
-    // first slot: the last one whose edge offset is <= b0 (256-way search rounds)
-    uint64_t lo = 0, hi = k;
-    while (hi - lo > 1) {
-      const uint64_t step = (hi - lo + 255) / 256;
-      const uint64_t probe = lo + (uint64_t)tid * step;
-      const bool le = probe < hi && eo[probe] <= b0;
-      const int cnt = __syncthreads_count(le);
-      lo = lo + (uint64_t)(cnt - 1) * step;
-      hi = lo + step < hi ? lo + step : hi;
+  const uint64_t windows = (E + kLoopThreads - 1) / kLoopThreads;
+  for (uint64_t w = blockIdx.x; w < windows; w += gridDim.x) {
+    const uint64_t base = w * kLoopThreads, last = base + kLoopThreads < E ? base + kLoopThreads - 1 : E - 1;
+    // Stage the slots this window touches: the one holding its first edge,
+    // then (every slot has >= 1 edge) at most kLoopThreads - 1 more.
+    const uint64_t sl = (uint64_t)wst[w] + tid;
+    const bool have = sl < k;
+    const uint32_t e = have ? eo[sl] : 0xffffffffu;
+    const uint32_t v = have ? q[sl] : 0u;
+    const bool mine = have && e <= last;
+    s->eo[tid] = e;
+    if (mine) {
+      s->v[tid] = v;
+      s->beg[tid] = off[v];
     }
-    uint64_t scur = lo;
-    for (uint64_t base = b0; base < b1; base += 256) {
-      const uint64_t last = base + 255 < b1 ? base + 255 : b1 - 1;
-      // Stage the slots this window touches.  scur holds the window's first
-      // edge and every slot has >= 1 edge, so at most 256 slots start at or
-      // before `last`; offset 257 tells whether the next window starts a slot.
-      const uint64_t sl = scur + tid;
-      const uint32_t e = sl < k ? eo[sl] : 0xffffffffu;
-      s_eo[tid] = e;
-      if (tid == 0) s_eo[256] = scur + 256 < k ? eo[scur + 256] : 0xffffffffu;
-      const int ns = __syncthreads_count(sl < k && e <= last);
-      if (tid < ns) {
-        const uint32_t v = q[scur + tid];
-        s_v[tid] = v;
-        s_beg[tid] = off[v];
+    const int ns = __syncthreads_count(mine);
+    const uint64_t t = base + tid;
+    bool add = false;
+    uint32_t u = 0, deg = 0;
+    if (t <= last) {
+      int a = 0, b = ns - 1;  // the last staged slot whose offset is <= t
+      while (a < b) {
+        const int mid = (a + b + 1) >> 1;
+        if (s->eo[mid] <= t)
+          a = mid;
+        else
+          b = mid - 1;
       }
-      __syncthreads();
-      const uint64_t t = base + tid;
-      bool add = false;
-      uint32_t u = 0, deg = 0;
-      if (t <= last) {
-        int a = 0, b = ns - 1;  // the last staged slot whose offset is <= t
-        while (a < b) {
-          const int mid = (a + b + 1) >> 1;
-          if (s_eo[mid] <= t)
-            a = mid;
-          else
-            b = mid - 1;
-        }
-        u = idx[s_beg[a] + (uint32_t)(t - s_eo[a])];
-        if (__ldcg(parents + u) == -1 && atomicCAS(parents + u, -1, (int32_t)s_v[a]) == -1) {
+      u = idx[s->beg[a] + (uint32_t)(t - s->eo[a])];
+      if (__ldcg(parents + u) == -1) {
+        // the degree is loaded beside the claim, not after it
+        const uint32_t d0 = __ldg(off + u), d1 = __ldg(off + u + 1);
+        if (atomicCAS(parents + u, -1, mark ? r : (int32_t)s->v[a]) == -1) {
           add = true;
           if (levels) levels[u] = r;
-          deg = off[u + 1] - off[u];
+          deg = d1 - d0;
         }
       }
-      block_append(add, u, deg, nq, neo, n, packed, zeros, nbits, s_scan, s_base);
-      // the slot holding edge last + 1: the next staged one if it starts there,
-      // else the last one staged (which runs past `last`)
-      scur += (s_eo[ns] == (uint32_t)(last + 1)) ? ns : ns - 1;
-      __syncthreads();
     }
+    block_append(add, u, deg, nq, neo, nwst, n, packed, zeros, nbits, s->scan, s->base);
+    __syncthreads();
   }
 }
 
 // Level 0's queue: the input frontier's vertices with out-edges, with offsets.
 __global__ void k_loop_seed(const uint32_t* in_q, uint64_t k, const uint32_t* off, uint32_t* q0, uint32_t* eo0,
-                            uint32_t n, LoopState* st) {
+                            uint32_t* wst0, uint32_t n, LoopState* st) {
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
   for (uint64_t i0 = (uint64_t)blockIdx.x * blockDim.x; i0 < k; i0 += stride) {  // warp-uniform trip count
     const uint64_t i = i0 + threadIdx.x;
@@ -272,21 +275,18 @@ __global__ void k_loop_seed(const uint32_t* in_q, uint64_t k, const uint32_t* of
       v = in_q[i];
       deg = off[v + 1] - off[v];
     }
-    loop_append(i < k && deg > 0, v, deg, q0, eo0, n, &st->slot[0].packed, &st->slot[0].zeros);
+    loop_append(i < k && deg > 0, v, deg, q0, eo0, wst0, n, &st->slot[0].packed, &st->slot[0].zeros);
   }
 }
 
-__global__ void __launch_bounds__(256) k_bfs_push_loop(const uint32_t* __restrict__ off,
-                                                       const uint32_t* __restrict__ idx, int32_t* parents,
-                                                       int32_t* levels, uint32_t* q0, uint32_t* q1, uint32_t* eo0,
-                                                       uint32_t* eo1, uint32_t n, LoopState* st, int32_t round0,
-                                                       unsigned long long threshold, int32_t max_levels,
-                                                       unsigned wait_budget) {
-  __shared__ uint32_t s_eo[257];
-  __shared__ uint32_t s_v[256];
-  __shared__ uint32_t s_beg[256];
-  __shared__ uint32_t s_scan[2][8];
-  __shared__ unsigned long long s_base[2];
+__global__ void __launch_bounds__(kLoopThreads) k_bfs_push_loop(const uint32_t* __restrict__ off,
+                                                                const uint32_t* __restrict__ idx, int32_t* parents,
+                                                                int32_t* levels, uint32_t* q0, uint32_t* q1,
+                                                                uint32_t* eo0, uint32_t* eo1, uint32_t* wst0,
+                                                                uint32_t* wst1, uint32_t n, LoopState* st,
+                                                                int32_t round0, unsigned long long threshold,
+                                                                int32_t max_levels, unsigned wait_budget) {
+  __shared__ PushShared s_push;
   __shared__ unsigned long long s_rd[5];
   __shared__ int s_ok;
   const int tid = threadIdx.x;
@@ -308,8 +308,8 @@ __global__ void __launch_bounds__(256) k_bfs_push_loop(const uint32_t* __restric
       st->trav += E;
     }
     const int32_t r = round0 + i;
-    push_level(off, idx, parents, levels, q, eo, nq, neo, k, E, n, r, &st->slot[nxt].packed, &st->slot[nxt].zeros,
-               nullptr, s_eo, s_v, s_beg, s_scan, s_base);
+    push_level(off, idx, parents, levels, q, eo, (i & 1) ? wst1 : wst0, nq, neo, (i & 1) ? wst0 : wst1, k, E, n, r, 0,
+               &st->slot[nxt].packed, &st->slot[nxt].zeros, nullptr, &s_push);
     target += gridDim.x;
     if (!grid_barrier(&st->bar, target, wait_budget, &s_ok, &st->slot[nxt], s_rd)) {
       if (tid == 0) atomicExch(&st->exit_reason, -1);
@@ -346,7 +346,7 @@ int bfs_device_levels(gg_graph_s* g, gg_frontier_s** F, int32_t* parents, int32_
   const int per_sm = occ.get(g->device, [dev = g->device]() {
     int coop = 0, b = 0;
     cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
-    if (!coop || cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_bfs_push_loop, 256, 0) != cudaSuccess || b < 1)
+    if (!coop || cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_bfs_push_loop, kLoopThreads, 0) != cudaSuccess || b < 1)
       return -1;
     return b;
   });
@@ -356,9 +356,11 @@ int bfs_device_levels(gg_graph_s* g, gg_frontier_s** F, int32_t* parents, int32_
   int rc = frontier_new(g, &fb);
   if (!rc) rc = frontier_ensure_queue(fa);
   if (!rc) rc = frontier_ensure_queue(fb);
-  DevBuf<uint32_t> eo0, eo1;
+  DevBuf<uint32_t> eo0, eo1, wst;
+  const uint64_t windows = g->m / kLoopThreads + 2;
   if (!rc) rc = eo0.alloc(g, n);
   if (!rc) rc = eo1.alloc(g, n);
+  if (!rc) rc = wst.alloc(g, 2 * windows);
   if (rc) {
     frontier_free(fa);
     frontier_free(fb);
@@ -369,25 +371,28 @@ int bfs_device_levels(gg_graph_s* g, gg_frontier_s** F, int32_t* parents, int32_
   cudaError_t e = cudaMemsetAsync(d_st, 0, sizeof(LoopState), g->stream);
   if (e == cudaSuccess) {
     k_loop_seed<<<generic_grid(g, in->dm), kGenericThreads, 0, g->stream>>>(in->d_queue, in->dm, g->out_off(),
-                                                                            fa->d_queue, eo0.p, n, d_st);
+                                                                            fa->d_queue, eo0.p, wst.p, n, d_st);
     e = cudaGetLastError();
   }
-  // a few CTAs per SM (4 unless set): sparse levels are small, and every CTA joins each barrier
-  const int grid = g->num_sms * std::min(per_sm, g->loop_ctas_per_sm > 0 ? g->loop_ctas_per_sm : 4);
+  // a few CTAs per SM (2 unless set): sparse levels are small, and every CTA joins each barrier
+  const int grid = g->num_sms * std::min(per_sm, g->loop_ctas_per_sm > 0 ? g->loop_ctas_per_sm : 2);
   const uint32_t* off = g->out_off();
   const uint32_t* idx = g->out_idx();
   uint32_t* q0 = fa->d_queue;
   uint32_t* q1 = fb->d_queue;
   uint32_t* e0 = eo0.p;
   uint32_t* e1 = eo1.p;
+  uint32_t* w0 = wst.p;
+  uint32_t* w1 = wst.p + windows;
   uint32_t nn = n;
   unsigned long long thr = threshold;
   int32_t cap = 1 << 20;
   unsigned budget = g->loop_wait_budget;
   void* args[] = {(void*)&off, (void*)&idx, (void*)&parents, (void*)&levels, (void*)&q0, (void*)&q1, (void*)&e0,
-                  (void*)&e1, (void*)&nn, (void*)&d_st, (void*)&round0, (void*)&thr, (void*)&cap, (void*)&budget};
+                  (void*)&e1, (void*)&w0, (void*)&w1, (void*)&nn, (void*)&d_st, (void*)&round0, (void*)&thr,
+                  (void*)&cap, (void*)&budget};
   if (e == cudaSuccess)
-    e = cudaLaunchCooperativeKernel((const void*)k_bfs_push_loop, grid, 256, args, 0, g->stream);
+    e = cudaLaunchCooperativeKernel((const void*)k_bfs_push_loop, grid, kLoopThreads, args, 0, g->stream);
   int rr = GG_OK;
   if (e == cudaSuccess) rr = read_small(g, &h, d_st);
   g->kernels += 2;
@@ -450,7 +455,7 @@ int bfs_device_levels(gg_graph_s* g, gg_frontier_s** F, int32_t* parents, int32_
 __device__ __noinline__ void bottom_up_level(const uint32_t* __restrict__ off, const uint32_t* __restrict__ ioff,
                                              const uint32_t* __restrict__ iidx, int32_t* parents, int32_t* levels,
                                              const uint32_t* bcur, uint32_t* bnxt, uint32_t n, int32_t r,
-                                             uint32_t* cnt, uint32_t* deg, int vec) {
+                                             int mark, uint32_t* cnt, uint32_t* deg, int vec) {
   const uint32_t lane = threadIdx.x & 31;
   const uint32_t stride = gridDim.x * blockDim.x;  // <= 2^31 threads
   uint32_t c = 0, dg = 0;
@@ -488,7 +493,7 @@ __device__ __noinline__ void bottom_up_level(const uint32_t* __restrict__ off, c
     bool act = false;
     if (v < n && pv == -1 && j0 < e1) {
       if ((bcur[s0 >> 5] >> (s0 & 31)) & 1u) {
-        parents[v] = (int32_t)s0;
+        parents[v] = mark ? r : (int32_t)s0;
         if (levels) levels[v] = r;
         act = true;
       } else if (vec) {
@@ -502,7 +507,7 @@ __device__ __noinline__ void bottom_up_level(const uint32_t* __restrict__ off, c
             if (e > j0 && e < e1 && ((bcur[ss[t] >> 5] >> (ss[t] & 31)) & 1u)) hit = t;
           }
           if (hit >= 0) {
-            parents[v] = (int32_t)ss[hit];
+            parents[v] = mark ? r : (int32_t)ss[hit];
             if (levels) levels[v] = r;
             act = true;
             break;
@@ -512,7 +517,7 @@ __device__ __noinline__ void bottom_up_level(const uint32_t* __restrict__ off, c
         for (uint32_t j = j0 + 1; j < e1; ++j) {
           const uint32_t s = iidx[j];
           if ((bcur[s >> 5] >> (s & 31)) & 1u) {
-            parents[v] = (int32_t)s;
+            parents[v] = mark ? r : (int32_t)s;
             if (levels) levels[v] = r;
             act = true;
             break;
@@ -539,11 +544,21 @@ __device__ __noinline__ void bottom_up_level(const uint32_t* __restrict__ off, c
   *deg = dg;
 }
 
-__global__ void k_bfs_full_seed(uint32_t start, const uint32_t* off, uint32_t* q0, uint32_t* eo0, uint32_t* bits0,
+// The start of a BFS in one pass: parents (and levels) unreached but for the
+// source, the bitmaps and the loop state clear, level 0's queue.
+__global__ void k_bfs_full_init(uint32_t n, uint32_t start, const uint32_t* off, int32_t* parents, int32_t* levels,
+                                uint32_t* q0, uint32_t* eo0, uint32_t* wst0, uint32_t* bits, uint32_t bit_words,
                                 LoopState* st) {
-  if (threadIdx.x == 0) {
-    const uint32_t d = off[start + 1] - off[start];
-    bits0[start >> 5] = 1u << (start & 31);
+  const uint64_t t0 = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (uint64_t)gridDim.x * blockDim.x;
+  for (uint64_t i = t0; i < n; i += stride) {
+    parents[i] = i == start ? (int32_t)start : -1;
+    if (levels) levels[i] = i == start ? 0 : -1;
+  }
+  for (uint64_t w = t0; w < bit_words; w += stride) bits[w] = w == (start >> 5) ? 1u << (start & 31) : 0u;
+  const uint32_t d = off[start + 1] - off[start];
+  for (uint64_t w = t0; w * kLoopThreads < d; w += stride) wst0[w] = 0;
+  if (t0 == 0) {
+    *st = LoopState{};
     q0[0] = start;
     eo0[0] = 0;
     if (d > 0)
@@ -553,8 +568,8 @@ __global__ void k_bfs_full_seed(uint32_t start, const uint32_t* off, uint32_t* q
   }
 }
 
-// Sums of five values over the CTA (blockDim.x == 256), returned to every thread.
-__device__ __forceinline__ void block_sum5(unsigned long long* v, unsigned long long (*s_red)[8]) {
+// Sums of five values over the CTA, returned to every thread.
+__device__ __forceinline__ void block_sum5(unsigned long long* v, unsigned long long (*s_red)[kLoopWarps]) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
   for (int j = 0; j < 5; ++j) v[j] = warp_sum(v[j]);
@@ -566,25 +581,19 @@ __device__ __forceinline__ void block_sum5(unsigned long long* v, unsigned long 
 #pragma unroll
   for (int j = 0; j < 5; ++j) {
     unsigned long long t = 0;
-    for (int w = 0; w < 8; ++w) t += s_red[j][w];
+    for (int w = 0; w < kLoopWarps; ++w) t += s_red[j][w];
     v[j] = t;
   }
 }
 
-__global__ void __launch_bounds__(256, 8) k_bfs_full(const uint32_t* __restrict__ off, const uint32_t* __restrict__ idx,
-                                                     const uint32_t* __restrict__ ioff,
-                                                     const uint32_t* __restrict__ iidx, int32_t* parents,
-                                                     int32_t* levels, uint32_t* q0, uint32_t* q1, uint32_t* eo0,
-                                                     uint32_t* eo1, uint32_t* bits, uint32_t wstride,
-                                                     unsigned long long* cta, uint32_t n, LoopState* st,
-                                                     int32_t round0, unsigned long long threshold,
-                                                     int32_t max_levels, unsigned wait_budget, int bu_vec) {
-  __shared__ uint32_t s_eo[257];
-  __shared__ uint32_t s_v[256];
-  __shared__ uint32_t s_beg[256];
-  __shared__ uint32_t s_scan[2][8];
-  __shared__ unsigned long long s_base[2];
-  __shared__ unsigned long long s_red[5][8];
+__global__ void __launch_bounds__(kLoopThreads, 2048 / kLoopThreads)
+    k_bfs_full(const uint32_t* __restrict__ off, const uint32_t* __restrict__ idx, const uint32_t* __restrict__ ioff,
+               const uint32_t* __restrict__ iidx, int32_t* parents, int32_t* levels, uint32_t* q0, uint32_t* q1,
+               uint32_t* eo0, uint32_t* eo1, uint32_t* wst0, uint32_t* wst1, uint32_t* bits, uint32_t wstride,
+               unsigned long long* cta, uint32_t n, LoopState* st, int32_t round0, unsigned long long threshold,
+               int32_t max_levels, unsigned wait_budget, int bu_vec, int mark) {
+  __shared__ PushShared s_push;
+  __shared__ unsigned long long s_red[5][kLoopWarps];
   __shared__ unsigned long long s_rd[5];
   __shared__ int s_ok;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -603,6 +612,7 @@ __global__ void __launch_bounds__(256, 8) k_bfs_full(const uint32_t* __restrict_
     const uint32_t* eo = (i & 1) ? eo1 : eo0;
     uint32_t* nq = (i & 1) ? q0 : q1;
     uint32_t* neo = (i & 1) ? eo0 : eo1;
+    uint32_t* nwst = (i & 1) ? wst0 : wst1;
     const uint32_t* bcur = bits + (size_t)cur * wstride;
     uint32_t* bnxt = bits + (size_t)nxt * wstride;
     uint32_t* bold = bits + (size_t)old * wstride;
@@ -622,7 +632,7 @@ __global__ void __launch_bounds__(256, 8) k_bfs_full(const uint32_t* __restrict_
     if (nk + E > threshold) {
       // bottom-up: one lane per destination, the first frontier in-neighbour wins
       uint32_t c32 = 0, dg32 = 0;
-      bottom_up_level(off, ioff, iidx, parents, levels, bcur, bnxt, n, r, &c32, &dg32, bu_vec);
+      bottom_up_level(off, ioff, iidx, parents, levels, bcur, bnxt, n, r, mark, &c32, &dg32, bu_vec);
       unsigned long long c = warp_sum((unsigned long long)c32), dg = warp_sum((unsigned long long)dg32);
       if (lane == 0) {
         s_red[0][warp] = c;
@@ -631,7 +641,7 @@ __global__ void __launch_bounds__(256, 8) k_bfs_full(const uint32_t* __restrict_
       __syncthreads();
       if (tid == 0) {
         unsigned long long tc = 0, td = 0;
-        for (int w = 0; w < 8; ++w) {
+        for (int w = 0; w < kLoopWarps; ++w) {
           tc += s_red[0][w];
           td += s_red[1][w];
         }
@@ -640,8 +650,8 @@ __global__ void __launch_bounds__(256, 8) k_bfs_full(const uint32_t* __restrict_
         if (blockIdx.x == 0) st->slot[nxt].rep = 1;
       }
     } else {
-      push_level(off, idx, parents, levels, q, eo, nq, neo, k, E, n, r, &st->slot[nxt].packed,
-                 &st->slot[nxt].zeros, bnxt, s_eo, s_v, s_beg, s_scan, s_base);
+      push_level(off, idx, parents, levels, q, eo, (i & 1) ? wst1 : wst0, nq, neo, nwst, k, E, n, r, mark,
+                 &st->slot[nxt].packed, &st->slot[nxt].zeros, bnxt, &s_push);
       if (blockIdx.x == 0 && tid == 0) st->slot[nxt].rep = 0;
     }
     target += gridDim.x;
@@ -700,7 +710,7 @@ __global__ void __launch_bounds__(256, 8) k_bfs_full(const uint32_t* __restrict_
       }
       block_sum5(t5, s_red);
       unsigned long long base_p = t5[0], base_d = t5[1];
-      // words in chunks of 256, one per thread, in order
+      // words in chunks of a CTA's threads, one per thread, in order
       for (uint32_t c0 = w0; c0 < w1; c0 += blockDim.x) {
         const uint32_t w = c0 + tid;
         const uint32_t x = w < w1 ? bnxt[w] : 0u;
@@ -715,9 +725,11 @@ __global__ void __launch_bounds__(256, 8) k_bfs_full(const uint32_t* __restrict_
             md += d;
           }
         }
-        uint32_t ep, ed, tpc, tdc;
-        block_scan2(mp, md, &ep, &ed, &tpc, &tdc, s_scan);
-        uint32_t slot = (uint32_t)base_p + ep, eoff = (uint32_t)base_d + ed;
+        // slots and edges of the words before (at most 32 kLoopThreads slots)
+        unsigned long long tot;
+        const unsigned long long ex = block_scan(((unsigned long long)mp << 32) | md, &tot, s_push.scan);
+        __syncthreads();
+        uint32_t slot = (uint32_t)base_p + (uint32_t)(ex >> 32), eoff = (uint32_t)base_d + (uint32_t)ex;
         y = x;
         while (y) {
           const uint32_t v = w * 32 + (__ffs(y) - 1);
@@ -726,12 +738,13 @@ __global__ void __launch_bounds__(256, 8) k_bfs_full(const uint32_t* __restrict_
           if (d) {
             nq[slot] = v;
             neo[slot] = eoff;
+            note_windows(nwst, slot, eoff, d);
             ++slot;
             eoff += d;
           }
         }
-        base_p += tpc;
-        base_d += tdc;
+        base_p += tot >> 32;
+        base_d += (uint32_t)tot;
       }
       // every CTA holds the totals (the next level's counters); the slot records them as well
       if (tid == 0) {
@@ -757,37 +770,52 @@ __global__ void __launch_bounds__(256, 8) k_bfs_full(const uint32_t* __restrict_
   }
 }
 
+// CTAs of the all-levels loop: every warp slot unless set (the bottom-up
+// levels are latency-bound), but no more than the graph has work for: a CTA
+// that only joins the barriers delays them (R-MAT-10: 53 us with every slot).
+static int full_grid(const gg_graph_s* g, int per_sm, uint64_t n, uint64_t m) {
+  const uint64_t slots =
+      (uint64_t)g->num_sms * std::min(per_sm, g->loop_ctas_per_sm > 0 ? g->loop_ctas_per_sm : 2048 / kLoopThreads);
+  return (int)std::min<uint64_t>(slots, std::max<uint64_t>(1, (n + m / 8) / (2 * kLoopThreads)));
+}
+
 // Enqueues every level of the BFS from `start` as one cooperative launch
-// (k_bfs_full) on the graph's stream and returns without waiting;
-// parents/levels hold the source's entries already (levels may be null).
-// bfs_device_full_result reads the outcome once the stream has passed it.
-int bfs_device_full(gg_graph_s* g, uint32_t start, int32_t* parents, int32_t* levels, uint64_t threshold) {
+// (k_bfs_full) on the graph's stream and returns without waiting.  `arena`
+// holds *parents and, when want_levels, *levels (n entries each) and the
+// loop's buffers.  bfs_device_full_begin_result queues the read-back of the
+// outcome, which bfs_device_full_result takes once the stream has passed it.
+int bfs_device_full(gg_graph_s* g, uint32_t start, bool want_levels, DevBuf<uint32_t>& arena, int32_t** parents,
+                    int32_t** levels, uint64_t threshold) {
   const uint32_t n = g->n;
   static DeviceOnce occ;
   const int per_sm = occ.get(g->device, [dev = g->device]() {
     int coop = 0, b = 0;
     cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
-    if (!coop || cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_bfs_full, 256, 0) != cudaSuccess || b < 1)
+    if (!coop || cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_bfs_full, kLoopThreads, 0) != cudaSuccess || b < 1)
       return -1;
     return b;
   });
   if (per_sm < 1) return fail(GG_ERR_UNSUPPORTED, "no cooperative launch of the BFS loop on this device");
-  // every warp slot unless set: the bottom-up levels are latency-bound
-  const int grid = g->num_sms * std::min(per_sm, g->loop_ctas_per_sm > 0 ? g->loop_ctas_per_sm : 8);
+  const int grid = full_grid(g, per_sm, n, g->m);
   const uint32_t words = (n + 31) / 32;
   const uint32_t wstride = (words + 31) & ~31u;  // 128-byte aligned bitmaps
-  DevBuf<uint32_t> q0, q1, eo0, eo1, bits;
-  DevBuf<unsigned long long> cta;
-  GG_TRY(q0.alloc(g, n));
-  GG_TRY(q1.alloc(g, n));
-  GG_TRY(eo0.alloc(g, n));
-  GG_TRY(eo1.alloc(g, n));
-  GG_TRY(bits.alloc(g, 3ull * wstride));
-  GG_TRY(cta.alloc(g, 3ull * grid));
+  const uint64_t na = ((uint64_t)n + 63) & ~63ull, wa = (g->m / kLoopThreads + 2 + 63) & ~63ull;
+  const uint64_t ca = ((uint64_t)grid * 6 + 63) & ~63ull;
+  GG_TRY(arena.alloc(g, na * (want_levels ? 6 : 5) + 2 * wa + 3ull * wstride + ca));
+  uint32_t* at = arena.p;
+  auto take = [&](uint64_t count) {
+    uint32_t* r = at;
+    at += count;
+    return r;
+  };
+  unsigned long long* cp = reinterpret_cast<unsigned long long*>(take(ca));
+  int32_t* par = reinterpret_cast<int32_t*>(take(na));
+  int32_t* lev = want_levels ? reinterpret_cast<int32_t*>(take(na)) : nullptr;
+  uint32_t *a0 = take(na), *a1 = take(na), *e0 = take(na), *e1 = take(na);
+  uint32_t *w0 = take(wa), *w1 = take(wa), *bp = take(3ull * wstride);
   LoopState* d_st = reinterpret_cast<LoopState*>(g->ws.d_loop);
-  GG_CUDA(cudaMemsetAsync(bits.p, 0, 4ull * 3 * wstride, g->stream));
-  GG_CUDA(cudaMemsetAsync(d_st, 0, sizeof(LoopState), g->stream));
-  k_bfs_full_seed<<<1, 32, 0, g->stream>>>(start, g->out_off(), q0.p, eo0.p, bits.p, d_st);
+  k_bfs_full_init<<<generic_grid(g, n), kGenericThreads, 0, g->stream>>>(n, start, g->out_off(), par, lev, a0, e0, w0,
+                                                                         bp, 3 * wstride, d_st);
   GG_CUDA(cudaGetLastError());
   const uint32_t* off = g->out_off();
   const uint32_t* idx = g->out_idx();
@@ -798,34 +826,33 @@ int bfs_device_full(gg_graph_s* g, uint32_t start, int32_t* parents, int32_t* le
   // memory, walk the CSC's own in-lists)
   if (g->early_kernel == 3 && !g->d_bu_idx && build_bu_index(g) != GG_OK) cudaGetLastError();
   const uint32_t* iidx = g->early_kernel == 3 && g->d_bu_idx ? g->d_bu_idx : g->in_idx();
-  uint32_t* a0 = q0.p;
-  uint32_t* a1 = q1.p;
-  uint32_t* e0 = eo0.p;
-  uint32_t* e1 = eo1.p;
-  uint32_t* bp = bits.p;
-  uint32_t ws = wstride;
-  unsigned long long* cp = cta.p;
-  uint32_t nn = n;
+  uint32_t ws = wstride, nn = n;
   int32_t round0 = 1;
   unsigned long long thr = threshold;
   int32_t cap = n < (uint32_t)INT32_MAX ? (int32_t)n + 1 : INT32_MAX;
   unsigned budget = g->loop_wait_budget;
-  int vec = g->early_kernel >= 2 ? 1 : 0;
-  void* args[] = {(void*)&off, (void*)&idx, (void*)&ioff, (void*)&iidx, (void*)&parents, (void*)&levels,
-                  (void*)&a0,  (void*)&a1,  (void*)&e0,   (void*)&e1,   (void*)&bp,      (void*)&ws,
-                  (void*)&cp,  (void*)&nn,  (void*)&d_st, (void*)&round0, (void*)&thr,   (void*)&cap,
-                  (void*)&budget, (void*)&vec};
-  GG_CUDA(cudaLaunchCooperativeKernel((const void*)k_bfs_full, grid, 256, args, 0, g->stream));
+  int vec = g->early_kernel >= 2 ? 1 : 0, mark = 0;
+  void* args[] = {(void*)&off, (void*)&idx, (void*)&ioff, (void*)&iidx, (void*)&par,  (void*)&lev,
+                  (void*)&a0,  (void*)&a1,  (void*)&e0,   (void*)&e1,   (void*)&w0,   (void*)&w1,
+                  (void*)&bp,  (void*)&ws,  (void*)&cp,   (void*)&nn,   (void*)&d_st, (void*)&round0,
+                  (void*)&thr, (void*)&cap, (void*)&budget, (void*)&vec, (void*)&mark};
+  GG_CUDA(cudaLaunchCooperativeKernel((const void*)k_bfs_full, grid, kLoopThreads, args, 0, g->stream));
   g->kernels += 2;
+  *parents = par;
+  *levels = lev;
   return GG_OK;
 }
 
-// The outcome of the BFS bfs_device_full enqueued (synchronises the stream):
-// *rounds, the number of edgeMap rounds (the last one finds nothing), *trav,
-// the out-degree sum of the frontiers processed.
+int bfs_device_full_begin_result(gg_graph_s* g) {
+  return read_small_begin(g, reinterpret_cast<const LoopState*>(g->ws.d_loop));
+}
+
+// The outcome of the BFS bfs_device_full enqueued, after the stream has passed
+// bfs_device_full_begin_result: *rounds, the number of edgeMap rounds (the last
+// one finds nothing), *trav, the out-degree sum of the frontiers processed.
 int bfs_device_full_result(gg_graph_s* g, int32_t* rounds, uint64_t* trav) {
   LoopState h{};
-  GG_TRY(read_small(g, &h, reinterpret_cast<const LoopState*>(g->ws.d_loop)));
+  read_small_end(g, &h);
   if (h.exit_reason < 0) return fail(GG_ERR_TIMEOUT, "BFS loop: a grid barrier wait ran out");
   if (h.exit_reason != 1)
     return fail(GG_ERR_CUDA, "BFS loop: stopped without an empty frontier (reason %d)", h.exit_reason);

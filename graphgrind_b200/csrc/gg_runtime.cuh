@@ -23,7 +23,13 @@ struct EventTimer {
     cudaEventRecord(a, s);
   }
   double stop() {
-    cudaEventRecord(b, s);
+    mark();
+    return elapsed();
+  }
+  // stop() in two halves: the end of the timed work, and its time once the
+  // caller has queued what else it wants on the stream
+  void mark() { cudaEventRecord(b, s); }
+  double elapsed() {
     cudaEventSynchronize(b);
     float ms = 0;
     cudaEventElapsedTime(&ms, a, b);
@@ -59,16 +65,27 @@ __global__ void k_put(T* dst, const T v) {
 }
 // Copies `count` values of T from device memory to `host` (any host memory)
 // after the graph's stream has reached this point; synchronises the stream.
+// In two halves for a caller with more to queue before it waits: begin queues
+// the copy into the mapped block, end reads it once the stream has passed.
 template <class T>
-int read_small(gg_graph_s* g, T* host, const T* dev, size_t count = 1) {
+int read_small_begin(gg_graph_s* g, const T* dev, size_t count = 1) {
   static_assert(sizeof(T) % 4 == 0, "control values are whole 32-bit words");
   const size_t bytes = sizeof(T) * count;
   if (bytes > kMapBytes) return fail(GG_ERR_INVALID_ARG, "control block of %zu bytes exceeds the mapped block", bytes);
   k_get_words<<<1, 128, 0, g->stream>>>(g->ws.d_map, reinterpret_cast<const uint32_t*>(dev), (uint32_t)(bytes / 4));
   GG_CUDA(cudaGetLastError());
   g->kernels++;
+  return GG_OK;
+}
+template <class T>
+void read_small_end(gg_graph_s* g, T* host, size_t count = 1) {
+  std::memcpy(host, g->ws.h_map, sizeof(T) * count);
+}
+template <class T>
+int read_small(gg_graph_s* g, T* host, const T* dev, size_t count = 1) {
+  GG_TRY(read_small_begin(g, dev, count));
   GG_CUDA(cudaStreamSynchronize(g->stream));
-  std::memcpy(host, g->ws.h_map, bytes);
+  read_small_end(g, host, count);
   return GG_OK;
 }
 // Writes one T to device memory in stream order (the value travels as a
@@ -245,7 +262,9 @@ int frontier_to_sparse(gg_frontier_s* f);
 void frontier_free(gg_frontier_s* f);
 int bfs_device_levels(gg_graph_s* g, gg_frontier_s** F, int32_t* parents, int32_t* levels, int32_t round0,
                       uint64_t threshold, int32_t* rounds, uint64_t* trav);
-int bfs_device_full(gg_graph_s* g, uint32_t start, int32_t* parents, int32_t* levels, uint64_t threshold);
+int bfs_device_full(gg_graph_s* g, uint32_t start, bool want_levels, DevBuf<uint32_t>& arena, int32_t** parents,
+                    int32_t** levels, uint64_t threshold);
+int bfs_device_full_begin_result(gg_graph_s* g);
 // The CSC's in-lists with each one's sources by descending out-degree (ties by
 // id), for BFS's bottom-up levels; built once per graph (g->d_bu_idx).
 int build_bu_index(gg_graph_s* g);

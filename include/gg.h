@@ -363,9 +363,10 @@ int gg_graph_set_dense_policy(gg_graph_t g, int32_t policy);
  *                         round.  Falls back to 0 by itself when the
  *                         driver refuses the capture; profiling also takes
  *                         the host loop
- *   GG_TUNE_LOOP_CTAS     CTAs per SM of those cooperative launches, 0..16
- *                         (0, the default: 4 for mode 1, 8 for mode 2; capped
- *                         by the kernel's occupancy)
+ *   GG_TUNE_LOOP_CTAS     CTAs (of 512 threads) per SM of those cooperative
+ *                         launches, 0..16 (0, the default: 2 for mode 1, 4 for
+ *                         mode 2; capped by the kernel's occupancy, and in
+ *                         mode 2 by the graph's size)
  *   GG_TUNE_CC_ALGO       0 (default): gg_components runs app/Components.C's
  *                         label propagation through edgeMap; 1: on symmetric
  *                         graphs, a union-find pass over the edges (each root
