@@ -12,7 +12,7 @@
 // window whose first edge it holds, so a CTA reaches its window's slots with
 // one load.  The barrier wait is bounded: on expiry the kernel records an error
 // and returns.
-#include "gg_runtime.cuh"
+#include "gg_loop.cuh"
 
 namespace gg {
 
@@ -24,30 +24,6 @@ namespace gg {
 // 1.59 / 2.16 ms with 256 / 512 / 1024 threads; R-MAT-22 0.53 / 0.52 / 0.53).
 constexpr int kLoopThreads = 512;
 constexpr int kLoopWarps = kLoopThreads / 32;
-
-// One frontier's counters; the loops keep three, by level mod 3.
-struct LoopSlot {
-  // queue form: (slots << 32) | out-edges; vertices with out-edges fill the
-  // queue from the front in edge-offset order
-  unsigned long long packed;
-  unsigned long long zeros;  // queue form: members without out-edges (not among the slots)
-  unsigned long long dcnt;   // bitmap form: members
-  unsigned long long ddeg;   // bitmap form: their out-degree sum
-  int32_t rep;               // 0 queue (and bitmap), 1 bitmap only
-  int32_t pad;
-};
-
-// State of a device level loop.  The counters are read after each grid
-// barrier by one thread per CTA (into shared memory); the barrier's arrival
-// word sits on a cache line of its own.
-struct LoopState {
-  LoopSlot slot[3];
-  unsigned long long trav;  // out-edges of the frontiers processed
-  alignas(128) unsigned int bar;  // barrier arrivals
-  int32_t levels_done;
-  int32_t exit_reason;  // 1 empty, 2 next level is dense (sparse loop), 3 level cap, -1 barrier timeout
-};
-static_assert(sizeof(LoopState) <= 64 * sizeof(unsigned long long), "loop state exceeds its workspace");
 
 __device__ __forceinline__ unsigned ld_acquire_u32(const unsigned* p) {
   unsigned v;
@@ -591,7 +567,7 @@ __global__ void __launch_bounds__(kLoopThreads, 2048 / kLoopThreads)
                const uint32_t* __restrict__ iidx, int32_t* parents, int32_t* levels, uint32_t* q0, uint32_t* q1,
                uint32_t* eo0, uint32_t* eo1, uint32_t* wst0, uint32_t* wst1, uint32_t* bits, uint32_t wstride,
                unsigned long long* cta, uint32_t n, LoopState* st, int32_t round0, unsigned long long threshold,
-               int32_t max_levels, unsigned wait_budget, int bu_vec, int mark) {
+               int32_t max_levels, unsigned wait_budget, int bu_vec, int mark, unsigned long long handover) {
   __shared__ PushShared s_push;
   __shared__ unsigned long long s_red[5][kLoopWarps];
   __shared__ unsigned long long s_rd[5];
@@ -663,10 +639,12 @@ __global__ void __launch_bounds__(kLoopThreads, 2048 / kLoopThreads)
     const unsigned long long npk = s_rd[0];
     const unsigned long long nk2 = nrep == 0 ? (npk >> 32) + s_rd[1] : s_rd[2];
     const unsigned long long nE = nrep == 0 ? npk & 0xffffffffull : s_rd[3];
-    if (nk2 == 0) {
+    // a frontier this small that no longer grows fast goes back to the caller
+    const bool give = nk2 + nE < handover && nE < 4 * E;
+    if (nk2 == 0 || give) {
       if (blockIdx.x == 0 && tid == 0) {
         st->levels_done = i + 1;
-        atomicCAS(&st->exit_reason, 0, 1);  // a timeout (-1) recorded by any CTA stays
+        atomicCAS(&st->exit_reason, 0, nk2 == 0 ? 1 : 4);  // a timeout (-1) recorded by any CTA stays
       }
       return;
     }
@@ -773,10 +751,21 @@ __global__ void __launch_bounds__(kLoopThreads, 2048 / kLoopThreads)
 // CTAs of the all-levels loop: every warp slot unless set (the bottom-up
 // levels are latency-bound), but no more than the graph has work for: a CTA
 // that only joins the barriers delays them (R-MAT-10: 53 us with every slot).
-static int full_grid(const gg_graph_s* g, int per_sm, uint64_t n, uint64_t m) {
-  const uint64_t slots =
-      (uint64_t)g->num_sms * std::min(per_sm, g->loop_ctas_per_sm > 0 ? g->loop_ctas_per_sm : 2048 / kLoopThreads);
-  return (int)std::min<uint64_t>(slots, std::max<uint64_t>(1, (n + m / 8) / (2 * kLoopThreads)));
+static int full_grid(int num_sms, int ctas_per_sm, uint64_t n, uint64_t m) {
+  return (int)std::min<uint64_t>((uint64_t)num_sms * ctas_per_sm,
+                                 std::max<uint64_t>(1, (n + m / 8) / (2 * kLoopThreads)));
+}
+
+// CTAs per SM that k_bfs_full can have resident in a cooperative launch; -1 if none.
+static int full_occupancy(int device) {
+  static DeviceOnce occ;
+  return occ.get(device, [device]() {
+    int coop = 0, b = 0;
+    cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device);
+    if (!coop || cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_bfs_full, kLoopThreads, 0) != cudaSuccess || b < 1)
+      return -1;
+    return b;
+  });
 }
 
 // Enqueues every level of the BFS from `start` as one cooperative launch
@@ -787,16 +776,10 @@ static int full_grid(const gg_graph_s* g, int per_sm, uint64_t n, uint64_t m) {
 int bfs_device_full(gg_graph_s* g, uint32_t start, bool want_levels, DevBuf<uint32_t>& arena, int32_t** parents,
                     int32_t** levels, uint64_t threshold) {
   const uint32_t n = g->n;
-  static DeviceOnce occ;
-  const int per_sm = occ.get(g->device, [dev = g->device]() {
-    int coop = 0, b = 0;
-    cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
-    if (!coop || cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_bfs_full, kLoopThreads, 0) != cudaSuccess || b < 1)
-      return -1;
-    return b;
-  });
+  const int per_sm = full_occupancy(g->device);
   if (per_sm < 1) return fail(GG_ERR_UNSUPPORTED, "no cooperative launch of the BFS loop on this device");
-  const int grid = full_grid(g, per_sm, n, g->m);
+  const int ctas = std::min(per_sm, g->loop_ctas_per_sm > 0 ? g->loop_ctas_per_sm : 2048 / kLoopThreads);
+  const int grid = full_grid(g->num_sms, ctas, n, g->m);
   const uint32_t words = (n + 31) / 32;
   const uint32_t wstride = (words + 31) & ~31u;  // 128-byte aligned bitmaps
   const uint64_t na = ((uint64_t)n + 63) & ~63ull, wa = (g->m / kLoopThreads + 2 + 63) & ~63ull;
@@ -832,10 +815,11 @@ int bfs_device_full(gg_graph_s* g, uint32_t start, bool want_levels, DevBuf<uint
   int32_t cap = n < (uint32_t)INT32_MAX ? (int32_t)n + 1 : INT32_MAX;
   unsigned budget = g->loop_wait_budget;
   int vec = g->early_kernel >= 2 ? 1 : 0, mark = 0;
+  unsigned long long handover = 0;
   void* args[] = {(void*)&off, (void*)&idx, (void*)&ioff, (void*)&iidx, (void*)&par,  (void*)&lev,
                   (void*)&a0,  (void*)&a1,  (void*)&e0,   (void*)&e1,   (void*)&w0,   (void*)&w1,
                   (void*)&bp,  (void*)&ws,  (void*)&cp,   (void*)&nn,   (void*)&d_st, (void*)&round0,
-                  (void*)&thr, (void*)&cap, (void*)&budget, (void*)&vec, (void*)&mark};
+                  (void*)&thr, (void*)&cap, (void*)&budget, (void*)&vec, (void*)&mark, (void*)&handover};
   GG_CUDA(cudaLaunchCooperativeKernel((const void*)k_bfs_full, grid, kLoopThreads, args, 0, g->stream));
   g->kernels += 2;
   *parents = par;
@@ -858,6 +842,98 @@ int bfs_device_full_result(gg_graph_s* g, int32_t* rounds, uint64_t* trav) {
     return fail(GG_ERR_CUDA, "BFS loop: stopped without an empty frontier (reason %d)", h.exit_reason);
   *rounds = h.levels_done;
   *trav = h.trav;
+  return GG_OK;
+}
+
+// ================================================== many graphs side by side
+// The loop's buffers inside a union's arena.
+struct UnionBufs {
+  unsigned long long* cta;
+  LoopState* st;
+  uint32_t *q0, *q1, *eo0, *eo1, *wst0, *wst1, *bits;
+  uint32_t wstride;
+  uint64_t words;  // of the whole arena
+};
+
+static UnionBufs union_bufs(const UnionBfs& u) {
+  UnionBufs b{};
+  const uint64_t na = ((uint64_t)u.n + 63) & ~63ull, wa = (u.m / kLoopThreads + 2 + 63) & ~63ull;
+  b.wstride = ((u.n + 31) / 32 + 31) & ~31u;
+  uint32_t* at = u.arena;
+  auto take = [&](uint64_t count) {
+    uint32_t* r = at ? at + b.words : nullptr;
+    b.words += count;
+    return r;
+  };
+  b.st = reinterpret_cast<LoopState*>(take(128));
+  b.cta = reinterpret_cast<unsigned long long*>(take(((uint64_t)u.grid * 6 + 63) & ~63ull));
+  b.q0 = take(na);
+  b.q1 = take(na);
+  b.eo0 = take(na);
+  b.eo1 = take(na);
+  b.wst0 = take(wa);
+  b.wst1 = take(wa);
+  b.bits = take(3ull * b.wstride);
+  return b;
+}
+
+int union_bfs_prepare(UnionBfs& u, int device, int num_sms) {
+  const int per_sm = full_occupancy(device);
+  if (per_sm < 1) return fail(GG_ERR_UNSUPPORTED, "no cooperative launch of the BFS loop on this device");
+  u.grid = full_grid(num_sms, std::min(per_sm, 2048 / kLoopThreads), u.n, u.m);
+  GG_CUDA(cudaMalloc(&u.arena, 4 * union_bufs(u).words));
+  u.st = union_bufs(u).st;
+  return GG_OK;
+}
+
+void union_bfs_free(UnionBfs& u) {
+  cudaFree(u.arena);
+  u.arena = nullptr;
+}
+
+__global__ void k_union_init(uint32_t n, int32_t* levels, uint32_t* bits, uint32_t bit_words, LoopState* st) {
+  const uint64_t t0 = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (uint64_t)gridDim.x * blockDim.x;
+  for (uint64_t i = t0; i < n; i += stride) levels[i] = -1;
+  for (uint64_t w = t0; w < bit_words; w += stride) bits[w] = 0;
+  if (t0 == 0) *st = LoopState{};
+}
+
+__global__ void k_union_seed(const uint32_t* seeds, uint32_t count, const uint32_t* off, int32_t* levels, uint32_t n,
+                             uint32_t* q0, uint32_t* eo0, uint32_t* wst0, uint32_t* bits, LoopState* st) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  uint32_t v = 0, deg = 0;
+  if (i < count) {
+    v = seeds[i];
+    deg = off[v + 1] - off[v];
+    levels[v] = 0;
+    atomicOr(bits + (v >> 5), 1u << (v & 31));
+  }
+  loop_append(i < count, v, deg, q0, eo0, wst0, n, &st->slot[0].packed, &st->slot[0].zeros);
+}
+
+int union_bfs_enqueue(const UnionBfs& u, cudaStream_t s, int num_sms, const uint32_t* seeds, uint32_t count) {
+  const UnionBufs b = union_bufs(u);
+  k_union_init<<<num_sms * 8, kGenericThreads, 0, s>>>(u.n, u.levels, b.bits, 3 * b.wstride, b.st);
+  k_union_seed<<<(count + 255) / 256, 256, 0, s>>>(seeds, count, u.off, u.levels, u.n, b.q0, b.eo0, b.wst0, b.bits,
+                                                   b.st);
+  GG_CUDA(cudaGetLastError());
+  int32_t* lev = u.levels;
+  int32_t* none = nullptr;
+  uint32_t ws = b.wstride, nn = u.n;
+  int32_t round0 = 1, cap = u.n < (uint32_t)INT32_MAX ? (int32_t)u.n + 1 : INT32_MAX;
+  unsigned long long thr = u.m / 20;  // edgeMap's m/20, over the union
+  unsigned budget = kWaitBudget;
+  int vec = 1, mark = 1;
+  // A level of the whole GPU costs about 10 us, a level inside one CTA per
+  // graph about 2.5 us a window: below a window of edges per graph the second
+  // is the faster one (256 R-MAT graphs: 0.62 ms with 2048 edges per graph, 0.56 with
+  // 512 and with 128).
+  unsigned long long handover = (unsigned long long)kLoopThreads * count;
+  void* args[] = {(void*)&u.off,  (void*)&u.idx,  (void*)&u.ioff,   (void*)&u.iidx, (void*)&lev,  (void*)&none,
+                  (void*)&b.q0,   (void*)&b.q1,   (void*)&b.eo0,    (void*)&b.eo1,  (void*)&b.wst0, (void*)&b.wst1,
+                  (void*)&b.bits, (void*)&ws,     (void*)&b.cta,    (void*)&nn,     (void*)&b.st, (void*)&round0,
+                  (void*)&thr,    (void*)&cap,    (void*)&budget,   (void*)&vec,    (void*)&mark, (void*)&handover};
+  GG_CUDA(cudaLaunchCooperativeKernel((const void*)k_bfs_full, u.grid, kLoopThreads, args, 0, s));
   return GG_OK;
 }
 

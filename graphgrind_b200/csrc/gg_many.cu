@@ -1,24 +1,36 @@
-// Many graphs in one launch: BFS over a batch of independent graphs of uneven
-// size.  All graphs live in one device arena; a persistent kernel's CTAs take
-// whole graphs from a device work queue (largest first) and run the
-// level-synchronous top-down traversal of app/BFS.C:77-101 inside the CTA,
-// with the frontier's edges load-balanced across the CTA's threads by a
-// block prefix sum over the frontier's degrees.  The launch sequence is
-// captured once as a CUDA graph and replayed.
+// Many graphs in one call: BFS over a batch of independent graphs of uneven
+// size.  The graphs live in one device arena as one union graph (vertices and
+// edges numbered consecutively), which the all-levels BFS loop traverses with
+// every CTA of the GPU on every level, top-down or bottom-up (gg_loop.cu): a
+// level's edges are spread over the GPU whatever graph they belong to, where
+// one CTA per graph would leave the GPU waiting for the largest one (256
+// R-MAT graphs of scale 10-16, 90M edges: 8.5 ms, of which the largest graph
+// alone).  Once the frontier is small and no longer grows, a persistent kernel
+// takes over, whose CTAs take whole graphs from a device work queue (largest
+// first) and finish each inside the CTA without grid barriers: its
+// level-synchronous top-down traversal of app/BFS.C:77-101 balances a
+// frontier's edges over the CTA's threads by a block prefix sum over the
+// frontier's degrees.  Batches past 2^31 vertices or 2^32 edges run in that
+// kernel alone.  The launch sequence is captured once as a CUDA graph and
+// replayed.
+#include <cub/cub.cuh>
+
 #include <algorithm>
 #include <mutex>
 #include <numeric>
 #include <unordered_set>
 #include <vector>
 
-#include "gg_runtime.cuh"
+#include "gg_loop.cuh"
 
+// Graph i's vertices are vfirst .. vfirst + n - 1 in the arenas: the union's
+// ids, or 0 .. n - 1 where the batch is too large for one union graph.
 struct BatchDesc {
-  uint64_t off_base;  // first offset of the graph in the offsets arena (n+1 entries)
-  uint64_t idx_base;  // first edge of the graph in the index arena
+  uint64_t off_base;  // the offset of the graph's first vertex in the offsets arena
+  uint64_t idx_base;  // where the offsets count from in the index arena
   uint64_t lev_base;  // first level slot of the graph
   uint32_t n;
-  uint32_t pad;
+  uint32_t vfirst;
 };
 
 struct gg_graph_batch_s {
@@ -28,13 +40,17 @@ struct gg_graph_batch_s {
   uint64_t total_n = 0, total_m = 0;
   uint32_t max_n = 0;
   std::vector<uint64_t> firsts;
+  bool whole = false;  // one union graph (else local ids, one CTA per graph)
+  int num_sms = 0;
+  gg::UnionBfs uni;
+  uint32_t *d_ioff = nullptr, *d_iidx = nullptr;
   uint32_t *d_off = nullptr, *d_idx = nullptr, *d_order = nullptr, *d_src = nullptr, *d_scratch = nullptr;
   BatchDesc* d_desc = nullptr;
   int32_t* d_levels = nullptr;
   unsigned long long* d_ctr = nullptr;  // [0] work ticket, [1] edges traversed
   uint32_t* h_src = nullptr;            // pinned
   int32_t* h_levels = nullptr;          // pinned
-  unsigned long long* h_ctr = nullptr;  // pinned
+  unsigned long long* h_ctr = nullptr;  // pinned: the counters, then the union loop's state
   int grid = 0;
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
@@ -58,12 +74,16 @@ __global__ void __launch_bounds__(kBatchThreads) k_batch_bfs(const BatchDesc* __
                                                               const uint32_t* __restrict__ idx, int32_t* levels,
                                                               const uint32_t* __restrict__ src,
                                                               unsigned long long* ctr, uint32_t* scratch,
-                                                              uint64_t stride) {
+                                                              uint64_t stride, const gg::LoopState* st) {
   __shared__ int32_t s_graph;
   __shared__ uint32_t s_scan[kBatchThreads + 1];
   __shared__ uint32_t s_beg[kBatchThreads];
   __shared__ uint32_t s_warp[32];
   __shared__ uint32_t s_nq;
+  // st: the union loop ran first, and either finished or left the vertices of
+  // level levels_done as the frontier
+  if (st && st->exit_reason != 4) return;
+  const int32_t level0 = st ? st->levels_done : 0;
   const int tid = threadIdx.x, lane = tid & 31;
   const uint32_t lanemask_lt = (1u << lane) - 1u;
   uint32_t* qa = scratch + (uint64_t)blockIdx.x * 2 * stride;
@@ -80,17 +100,42 @@ __global__ void __launch_bounds__(kBatchThreads) k_batch_bfs(const BatchDesc* __
     const BatchDesc d = desc[gi];
     const uint32_t* go = off + d.off_base;
     const uint32_t* gx = idx + d.idx_base;
-    int32_t* lev = levels + d.lev_base;
-    for (uint32_t v = tid; v < d.n; v += kBatchThreads) lev[v] = -1;
-    __syncthreads();
-    const uint32_t s = src[gi];
-    if (tid == 0) {
-      lev[s] = 0;
-      qa[0] = s;
-    }
+    int32_t* lev = levels + d.lev_base;  // lev, go and the queues: local vertices; gx: arena ids
     uint32_t qn = 1;
-    int32_t r = 0;
-    __syncthreads();
+    int32_t r = level0;
+    if (st) {  // the frontier is what the levels say
+      if (tid == 0) s_nq = 0;
+      __syncthreads();
+      for (uint32_t v0 = tid; v0 - tid < d.n; v0 += 8 * kBatchThreads) {  // 8 loads in flight per thread
+        int32_t l[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) l[u] = v0 + u * kBatchThreads < d.n ? __ldcg(lev + v0 + u * kBatchThreads) : -1;
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+          const bool add = l[u] == level0;
+          const uint32_t bal = __ballot_sync(0xffffffffu, add);
+          if (bal) {
+            const int leader = __ffs(bal) - 1;
+            uint32_t base = 0;
+            if (lane == leader) base = atomicAdd(&s_nq, (uint32_t)__popc(bal));
+            base = __shfl_sync(0xffffffffu, base, leader);
+            if (add) qa[base + __popc(bal & lanemask_lt)] = v0 + u * kBatchThreads;
+          }
+        }
+      }
+      __syncthreads();
+      qn = s_nq;
+      __syncthreads();
+    } else {
+      for (uint32_t v = tid; v < d.n; v += kBatchThreads) lev[v] = -1;
+      __syncthreads();
+      const uint32_t s = src[gi];
+      if (tid == 0) {
+        lev[s] = 0;
+        qa[0] = s;
+      }
+      __syncthreads();
+    }
     while (qn > 0) {
       ++r;
       if (tid == 0) s_nq = 0;
@@ -123,7 +168,7 @@ __global__ void __launch_bounds__(kBatchThreads) k_batch_bfs(const BatchDesc* __
               else
                 hi = mid - 1;
             }
-            u = gx[s_beg[lo] + (t - s_scan[lo])];
+            u = gx[s_beg[lo] + (t - s_scan[lo])] - d.vfirst;
             if (__ldcg(lev + u) < 0) add = atomicCAS(lev + u, -1, r) == -1;
           }
           const uint32_t bal = __ballot_sync(0xffffffffu, add);
@@ -151,8 +196,11 @@ static void batch_release(gg_graph_batch_s* b) {
   if (!b) return;
   if (b->exec) cudaGraphExecDestroy(b->exec);
   if (b->graph) cudaGraphDestroy(b->graph);
+  gg::union_bfs_free(b->uni);
   cudaFree(b->d_off);
   cudaFree(b->d_idx);
+  cudaFree(b->d_ioff);
+  cudaFree(b->d_iidx);
   cudaFree(b->d_order);
   cudaFree(b->d_src);
   cudaFree(b->d_scratch);
@@ -166,23 +214,87 @@ static void batch_release(gg_graph_batch_s* b) {
   delete b;
 }
 
+// Global ids for every edge of the union (CTAs over graphs).
+__global__ void k_batch_globalise(const BatchDesc* desc, const uint64_t* edge_first, int32_t count, uint32_t* idx) {
+  for (int32_t i = blockIdx.x; i < count; i += gridDim.x) {
+    const uint32_t base = desc[i].vfirst;
+    for (uint64_t e = edge_first[i] + threadIdx.x; e < edge_first[i + 1]; e += blockDim.x) idx[e] += base;
+  }
+}
+
+// The source of every out-edge, one warp per vertex.
+__global__ void k_batch_src(uint32_t n, const uint32_t* off, uint32_t* src) {
+  const uint64_t w0 = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+  for (uint64_t v = w0; v < n; v += nw)
+    for (uint32_t e = off[v] + (threadIdx.x & 31); e < off[v + 1]; e += 32) src[e] = (uint32_t)v;
+}
+
+// In-offsets from the edges' destinations in ascending order.
+__global__ void k_batch_in_off(uint64_t m, uint32_t n, const uint32_t* dst, uint32_t* ioff) {
+  for (uint64_t e = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; e <= m; e += (uint64_t)gridDim.x * blockDim.x) {
+    const uint32_t from = e ? dst[e - 1] + 1 : 0, to = e < m ? dst[e] : n;  // vertices whose in-edges begin at e
+    for (uint64_t v = from; v <= to; ++v) ioff[v] = (uint32_t)e;
+  }
+}
+
+// The union's in-edges, for the bottom-up levels: a stable sort by
+// destination, so in-lists stay in source order.
+static int batch_in_edges(gg_graph_batch_s* b, uint32_t n) {
+  const uint64_t m = b->total_m;
+  GG_CUDA(cudaMalloc(&b->d_ioff, 4 * ((uint64_t)n + 1)));
+  GG_CUDA(cudaMalloc(&b->d_iidx, 4 * (m + 16)));
+  GG_CUDA(cudaMemsetAsync(b->d_iidx + m, 0, 64, b->stream));
+  struct Hold {
+    void* p[3] = {nullptr, nullptr, nullptr};
+    ~Hold() {
+      for (void* q : p) cudaFree(q);
+    }
+  } h;
+  const uint64_t me = std::max<uint64_t>(m, 1);
+  GG_CUDA(cudaMalloc(&h.p[0], 4 * me));
+  GG_CUDA(cudaMalloc(&h.p[1], 4 * me));
+  uint32_t *src = static_cast<uint32_t*>(h.p[0]), *dst = static_cast<uint32_t*>(h.p[1]);
+  const int grid = b->num_sms * 8;
+  int bits = 1;
+  while (bits < 32 && (n - 1) >> bits) ++bits;
+  if (m) {
+    k_batch_src<<<grid, 256, 0, b->stream>>>(n, b->d_off, src);
+    GG_CUDA(cudaGetLastError());
+    size_t temp = 0;
+    GG_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, temp, b->d_idx, dst, src, b->d_iidx, m, 0, bits, b->stream));
+    GG_CUDA(cudaMalloc(&h.p[2], std::max<size_t>(temp, 1)));
+    GG_CUDA(cub::DeviceRadixSort::SortPairs(h.p[2], temp, b->d_idx, dst, src, b->d_iidx, m, 0, bits, b->stream));
+  }
+  k_batch_in_off<<<grid, 256, 0, b->stream>>>(m, n, dst, b->d_ioff);
+  GG_CUDA(cudaGetLastError());
+  GG_CUDA(cudaStreamSynchronize(b->stream));
+  return GG_OK;
+}
+
 static int batch_build(int32_t count, const gg_host_graph* graphs, gg_graph_batch_s* b) {
   b->count = count;
   std::vector<BatchDesc> desc(count);
-  uint64_t offs = 0;
   for (int32_t i = 0; i < count; ++i) {
     const gg_host_graph& h = graphs[i];
     if (h.n == 0 || !h.offsets || (h.m && !h.indices) || h.offsets[h.n] != h.m)
       return fail(GG_ERR_INVALID_ARG, "gg_batch_create: graph %d is malformed", i);
-    desc[i] = BatchDesc{offs, b->total_m, b->total_n, h.n, 0};
     b->firsts.push_back(b->total_n);
-    offs += (uint64_t)h.n + 1;
     b->total_m += h.m;
     b->total_n += h.n;
     b->max_n = std::max(b->max_n, h.n);
   }
+  b->whole = b->total_n < (1ull << 31) && b->total_m < (1ull << 32) - 64;
+  std::vector<uint64_t> edge_first(count + 1, 0);
+  for (int32_t i = 0; i < count; ++i) edge_first[i + 1] = edge_first[i] + graphs[i].m;
+  for (int32_t i = 0; i < count; ++i) {
+    const uint64_t v0 = b->firsts[i];
+    desc[i] = b->whole ? BatchDesc{v0, 0, v0, graphs[i].n, (uint32_t)v0}
+                       : BatchDesc{v0 + (uint64_t)i, edge_first[i], v0, graphs[i].n, 0};
+  }
+  const uint64_t offs = b->whole ? b->total_n + 1 : b->total_n + count;
   GG_CUDA(cudaGetDevice(&b->device));
   GG_CUDA(cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking));
+  GG_CUDA(cudaDeviceGetAttribute(&b->num_sms, cudaDevAttrMultiProcessorCount, b->device));
   GG_CUDA(cudaMalloc(&b->d_off, 4 * offs));
   GG_CUDA(cudaMalloc(&b->d_idx, 4 * std::max<uint64_t>(b->total_m, 1)));
   GG_CUDA(cudaMalloc(&b->d_levels, 4 * b->total_n));
@@ -190,35 +302,78 @@ static int batch_build(int32_t count, const gg_host_graph* graphs, gg_graph_batc
   GG_CUDA(cudaMalloc(&b->d_order, 4 * count));
   GG_CUDA(cudaMalloc(&b->d_src, 4 * count));
   GG_CUDA(cudaMalloc(&b->d_ctr, 16));
-  for (int32_t i = 0; i < count; ++i) {
-    const gg_host_graph& h = graphs[i];
-    GG_CUDA(cudaMemcpy(b->d_off + desc[i].off_base, h.offsets, 4 * ((uint64_t)h.n + 1), cudaMemcpyHostToDevice));
-    if (h.m) GG_CUDA(cudaMemcpy(b->d_idx + desc[i].idx_base, h.indices, 4 * h.m, cudaMemcpyHostToDevice));
+  GG_CUDA(cudaMemcpy(b->d_desc, desc.data(), sizeof(BatchDesc) * count, cudaMemcpyHostToDevice));
+  {
+    std::vector<uint32_t> off(offs);
+#pragma omp parallel for schedule(dynamic, 8)
+    for (int32_t i = 0; i < count; ++i) {
+      const gg_host_graph& h = graphs[i];
+      const uint32_t base = b->whole ? (uint32_t)edge_first[i] : 0u;
+      for (uint64_t v = 0; v < (uint64_t)h.n + (b->whole ? 0 : 1); ++v) off[desc[i].off_base + v] = h.offsets[v] + base;
+    }
+    if (b->whole) off[b->total_n] = (uint32_t)b->total_m;
+    GG_CUDA(cudaMemcpy(b->d_off, off.data(), 4 * offs, cudaMemcpyHostToDevice));
+  }
+  for (int32_t i = 0; i < count; ++i)
+    if (graphs[i].m)
+      GG_CUDA(cudaMemcpy(b->d_idx + edge_first[i], graphs[i].indices, 4 * graphs[i].m, cudaMemcpyHostToDevice));
+  if (b->whole) {
+    uint64_t* d_first = nullptr;
+    GG_CUDA(cudaMalloc(&d_first, 8 * ((uint64_t)count + 1)));
+    struct Hold {
+      void* p;
+      ~Hold() { cudaFree(p); }
+    } hold{d_first};
+    GG_CUDA(cudaMemcpy(d_first, edge_first.data(), 8 * ((uint64_t)count + 1), cudaMemcpyHostToDevice));
+    k_batch_globalise<<<std::min(count, b->num_sms * 8), 256, 0, b->stream>>>(b->d_desc, d_first, count, b->d_idx);
+    GG_CUDA(cudaGetLastError());
+    GG_TRY(batch_in_edges(b, (uint32_t)b->total_n));
+    b->uni.off = b->d_off;
+    b->uni.idx = b->d_idx;
+    b->uni.ioff = b->d_ioff;
+    b->uni.iidx = b->d_iidx;
+    b->uni.levels = b->d_levels;
+    b->uni.n = (uint32_t)b->total_n;
+    b->uni.m = b->total_m;
+    GG_TRY(union_bfs_prepare(b->uni, b->device, b->num_sms));
   }
   std::vector<uint32_t> order(count);
   std::iota(order.begin(), order.end(), 0u);
   std::stable_sort(order.begin(), order.end(), [&](uint32_t x, uint32_t y) { return graphs[x].m > graphs[y].m; });
-  GG_CUDA(cudaMemcpy(b->d_desc, desc.data(), sizeof(BatchDesc) * count, cudaMemcpyHostToDevice));
   GG_CUDA(cudaMemcpy(b->d_order, order.data(), 4 * count, cudaMemcpyHostToDevice));
-  int sms = 0, per_sm = 0;
-  GG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, b->device));
+  int per_sm = 0;
   GG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batch_bfs, kBatchThreads, 0));
-  b->grid = std::max(1, std::min(count, sms * std::max(per_sm, 1)));
+  b->grid = std::max(1, std::min(count, b->num_sms * std::max(per_sm, 1)));
   GG_CUDA(cudaMalloc(&b->d_scratch, 8ull * b->max_n * b->grid));
   GG_CUDA(cudaMallocHost(&b->h_src, 4 * count));
   GG_CUDA(cudaMallocHost(&b->h_levels, 4 * b->total_n));
-  GG_CUDA(cudaMallocHost(&b->h_ctr, 16));
-  // the replayed sequence: sources up, counters reset, persistent traversal, levels and counters down
+  GG_CUDA(cudaMallocHost(&b->h_ctr, 16 + sizeof(LoopState)));
+  // the replayed sequence: sources up, counters reset, traversal, counters down
   GG_CUDA(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
   cudaMemcpyAsync(b->d_src, b->h_src, 4 * count, cudaMemcpyHostToDevice, b->stream);
   cudaMemsetAsync(b->d_ctr, 0, 16, b->stream);
+  if (b->whole) GG_TRY(union_bfs_enqueue(b->uni, b->stream, b->num_sms, b->d_src, (uint32_t)count));
   k_batch_bfs<<<b->grid, kBatchThreads, 0, b->stream>>>(b->d_desc, b->d_order, count, b->d_off, b->d_idx,
-                                                          b->d_levels, b->d_src, b->d_ctr, b->d_scratch, b->max_n);
-  cudaMemcpyAsync(b->h_levels, b->d_levels, 4 * b->total_n, cudaMemcpyDeviceToHost, b->stream);
+                                                          b->d_levels, b->d_src, b->d_ctr, b->d_scratch, b->max_n,
+                                                          b->whole ? b->uni.st : nullptr);
   cudaMemcpyAsync(b->h_ctr, b->d_ctr, 16, cudaMemcpyDeviceToHost, b->stream);
+  if (b->whole)
+    cudaMemcpyAsync(b->h_ctr + 2, b->uni.st, sizeof(LoopState), cudaMemcpyDeviceToHost, b->stream);
   GG_CUDA(cudaStreamEndCapture(b->stream, &b->graph));
   GG_CUDA(cudaGraphInstantiate(&b->exec, b->graph, 0));
   return GG_OK;
+}
+
+// Whether bytes [p, p + bytes) are page-locked host memory at both ends (a
+// copy from the device then needs no staging).
+static bool pinned_range(const void* p, size_t bytes) {
+  if (bytes == 0) return false;
+  cudaPointerAttributes a{}, z{};
+  const bool ok = cudaPointerGetAttributes(&a, p) == cudaSuccess && a.type == cudaMemoryTypeHost &&
+                  cudaPointerGetAttributes(&z, static_cast<const char*>(p) + bytes - 1) == cudaSuccess &&
+                  z.type == cudaMemoryTypeHost;
+  if (!ok) cudaGetLastError();
+  return ok;
 }
 
 }  // namespace gg
@@ -277,18 +432,24 @@ int gg_batch_bfs(gg_graph_batch_t b, const uint32_t* sources, int32_t* levels, g
     const uint64_t n = (i + 1 < b->count ? b->firsts[i + 1] : b->total_n) - b->firsts[i];
     if (sources[i] >= n) return fail(GG_ERR_INVALID_ARG, "gg_batch_bfs: source %u of graph %d out of range", sources[i], i);
   }
-  std::copy(sources, sources + b->count, b->h_src);
+  for (int32_t i = 0; i < b->count; ++i) b->h_src[i] = sources[i] + (b->whole ? (uint32_t)b->firsts[i] : 0u);
   EventTimer tm(b->stream);
   GG_CUDA(cudaGraphLaunch(b->exec, b->stream));
+  int32_t* down = levels && pinned_range(levels, 4 * b->total_n) ? levels : b->h_levels;
+  GG_CUDA(cudaMemcpyAsync(down, b->d_levels, 4 * b->total_n, cudaMemcpyDeviceToHost, b->stream));
   const double ms = tm.stop();
   GG_CUDA(cudaStreamSynchronize(b->stream));
   GG_CUDA(cudaGetLastError());
-  if (levels) std::copy(b->h_levels, b->h_levels + b->total_n, levels);
+  const LoopState* loop = reinterpret_cast<const LoopState*>(b->h_ctr + 2);
+  if (b->whole && loop->exit_reason < 0) return fail(GG_ERR_TIMEOUT, "gg_batch_bfs: a grid barrier wait ran out");
+  if (b->whole && loop->exit_reason != 1 && loop->exit_reason != 4)
+    return fail(GG_ERR_CUDA, "gg_batch_bfs: stopped without an empty frontier (reason %d)", loop->exit_reason);
+  if (levels && down != levels) std::copy(b->h_levels, b->h_levels + b->total_n, levels);
   if (st) {
     st->ms = ms;
     st->rounds = 1;
-    st->edges_traversed = b->h_ctr[1];
-    st->kernels = 1;
+    st->edges_traversed = b->h_ctr[1] + (b->whole ? loop->trav : 0);
+    st->kernels = b->whole ? 4 : 1;
   }
   return GG_OK;
 }

@@ -602,12 +602,15 @@ int gg_batch_destroy(gg_graph_batch_t b);
  * receives each graph's first slot in the level output. */
 int gg_batch_info(gg_graph_batch_t b, uint64_t* total_vertices, uint64_t* total_edges, uint64_t* firsts);
 /* BFS from sources[i] in graph i for every graph (app/BFS.C:77-101 levels),
- * in one persistent launch whose CTAs take graphs, largest first, from a
- * device work queue and traverse each inside the CTA.  levels: host array of
- * total_vertices int32 (may be NULL), graph i's at firsts[i], -1 unreached.
- * The sequence source upload -> traversal -> level download is a CUDA graph
- * captured at gg_batch_create and replayed by every call; st->ms is its
- * device time, st->edges_traversed the sum over graphs of gg_bfs's count. */
+ * as one union graph whose levels run on the whole GPU, top-down or bottom-up;
+ * once the frontier is small, persistent CTAs take whole graphs, largest
+ * first, from a device work queue and finish each inside the CTA (a batch past
+ * 2^31 vertices or 2^32 edges runs in that form alone).  levels: host array of
+ * total_vertices int32 (may be NULL), graph i's at firsts[i], -1 unreached;
+ * page-locked memory is filled without staging.  The sequence source upload ->
+ * traversal is a CUDA graph captured at gg_batch_create and replayed by every
+ * call; st->ms is its device time with the level download, st->edges_traversed
+ * the sum over graphs of gg_bfs's count. */
 int gg_batch_bfs(gg_graph_batch_t b, const uint32_t* sources, int32_t* levels, gg_run_stats* st);
 
 /* ==================================================== differentiation */
