@@ -103,15 +103,84 @@ __global__ void __launch_bounds__(256) k_ppr_pull(const uint32_t* idx, const uin
   }
 }
 
-// Zero the S rows that receive partial sums (rows crossing a block boundary).
-__global__ void k_zero_rows(const uint32_t* rows_list, uint32_t count, float* S, uint32_t k) {
-  const uint64_t total = (uint64_t)count * k;
-  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (uint64_t)gridDim.x * blockDim.x)
-    S[(uint64_t)rows_list[i / k] * k + (i % k)] = 0.f;
+// The rows that cross a 256-edge block boundary (they receive partial sums):
+// row_list[0 .. *count).  The row that continues into block b is listed by the
+// first block it continues into.
+__global__ void k_boundary_rows(const uint32_t* head, const uint32_t* blk, const uint32_t* rows, uint64_t nblocks,
+                                uint32_t* row_list, uint32_t* count) {
+  for (uint64_t b = 1 + (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; b < nblocks;
+       b += (uint64_t)gridDim.x * blockDim.x) {
+    const uint32_t h = blk[b];
+    if (!(head[b * 8] & 1u) && h != blk[b - 1]) row_list[atomicAdd(count, 1u)] = rows[h - 1];
+  }
 }
 
-// Vertex pass: Y = d*S + (1-d)*T (S = 0 for vertices without in-edges), and
-// the next iteration's per-source rows XS = Y / outdeg.
+// Zero the S rows that receive partial sums.
+__global__ void k_zero_rows(const uint32_t* row_list, const uint32_t* count, float* S, uint32_t k) {
+  const uint64_t total = (uint64_t)*count * k;
+  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (uint64_t)gridDim.x * blockDim.x)
+    S[(uint64_t)row_list[i / k] * k + (i % k)] = 0.f;
+}
+
+// tbits: the rows of T that are not all zero, one warp per row.
+__global__ void k_ppr_tbits(uint32_t n, uint32_t k, const float* T, uint32_t* tbits) {
+  const int lane = threadIdx.x & 31;
+  const uint64_t w0 = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+  for (uint64_t v = w0; v < n; v += nw) {
+    bool nz = false;
+    for (uint32_t c = lane; c < k; c += 32) nz |= T[v * k + c] != 0.f;
+    if (__any_sync(0xffffffffu, nz) && lane == 0) atomicOr(tbits + (v >> 5), 1u << (v & 31));
+  }
+}
+
+// One-hot T: the seeds' rows zeroed and marked (one warp per seed); the other rows are never read.
+__global__ void k_ppr_seed_rows(const uint32_t* seeds, uint32_t k, float* T, uint32_t* tbits) {
+  const uint32_t j = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  if (j >= k) return;
+  for (uint32_t c = lane; c < k; c += 32) T[(uint64_t)seeds[j] * k + c] = 0.f;
+  if (lane == 0) atomicOr(tbits + (seeds[j] >> 5), 1u << (seeds[j] & 31));
+}
+
+// Vertex pass of k = 2^ksh (32 or 64) columns, four per thread: y = d*S +
+// (1-d)*T, out = y / outdeg, the next iteration's scaled rows, or y itself
+// after the last one.  first: y = T, the rows the iterations start from.  What
+// bounds it is memory, so rows of T that hold only zeros (every row but the
+// seeds' of a one-hot T), marked by a clear bit, are not read, such a row
+// without in-edges stays at the zeros the first pass gave it, and only the
+// array the next step needs is written (64 columns, R-MAT-18: 74 us a pass
+// with all arrays and a division by k per value, 37 us now).
+__global__ void __launch_bounds__(256) k_ppr_rows(uint64_t total4, int ksh, const uint32_t* __restrict__ in_off,
+                                                  const uint32_t* __restrict__ out_off,
+                                                  const float* __restrict__ S, const float* __restrict__ T,
+                                                  const uint32_t* __restrict__ tbits, float damping, float* out,
+                                                  int first, int last) {
+  for (uint64_t q = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; q < total4; q += (uint64_t)gridDim.x * blockDim.x) {
+    const uint32_t v = (uint32_t)(q >> (ksh - 2));
+    const bool marked = test_bit(tbits, v);
+    if (!first && !marked && in_off[v + 1] == in_off[v]) continue;
+    float4 y = make_float4(0.f, 0.f, 0.f, 0.f);
+    const float4 t = marked ? reinterpret_cast<const float4*>(T)[q] : y;
+    if (first) {
+      y = t;
+    } else {
+      y = reinterpret_cast<const float4*>(S)[q];
+      y.x = damping * y.x + (1.f - damping) * t.x;
+      y.y = damping * y.y + (1.f - damping) * t.y;
+      y.z = damping * y.z + (1.f - damping) * t.z;
+      y.w = damping * y.w + (1.f - damping) * t.w;
+    }
+    if (!last) {
+      const uint32_t d = out_off[v + 1] - out_off[v];
+      const float df = (float)d;
+      y = d ? make_float4(y.x / df, y.y / df, y.z / df, y.w / df) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    reinterpret_cast<float4*>(out)[q] = y;
+  }
+}
+
+// One column (k = 1): the vertex pass after the engine's scalar pull, Y = d*S +
+// (1-d)*T (S = 0 for vertices without in-edges), and the next iteration's
+// per-source values XS = Y / outdeg.
 __global__ void k_ppr_vertex(uint32_t n, uint32_t k, const uint32_t* in_off, const uint32_t* out_off, const float* S,
                              const float* T, float damping, float* Y, float* XS, int write_y) {
   const uint64_t total = (uint64_t)n * k;
@@ -139,13 +208,42 @@ __global__ void k_ppr_init(uint32_t n, uint32_t k, const float* T, const uint32_
   }
 }
 
-// Rows whose in-edges cross a 256-edge block boundary (static per graph).
-static int boundary_rows(gg_graph_s* g, std::vector<uint32_t>& out) {
-  const uint32_t* off = g->transposed ? g->h_csr_off.data() : g->h_csc_off.data();
-  for (uint32_t v = 0; v < g->n; ++v) {
-    const uint32_t a = off[v], b = off[v + 1];
-    if (b > a && (a / kSegBlock) != ((b - 1) / kSegBlock)) out.push_back(v);
+// The iterations of k = 32 or 64 columns: T and its tbits hold the teleport
+// rows, XS and S are n x k buffers.  The result is left in XS.
+static int ppr_columns(gg_graph_s* g, uint32_t k, int32_t iters, float damping, const float* T, const uint32_t* tbits,
+                       float* XS, float* S) {
+  const uint64_t nblocks = (g->m + kSegBlock - 1) / kSegBlock, total4 = (uint64_t)g->n * k / 4;
+  const SegIndex& si = g->seg[g->transposed ? 1 : 0];
+  const int ksh = k == 64 ? 6 : 5, vgrid = generic_grid(g, total4);
+  const int pgrid = (int)std::max<uint64_t>(1, std::min<uint64_t>((nblocks + 7) / 8, (uint64_t)g->num_sms * 16));
+  DevBuf<uint32_t> brows;  // the count, then the rows
+  GG_TRY(brows.alloc(g, nblocks + 4));
+  GG_CUDA(cudaMemsetAsync(brows.p, 0, 4, g->stream));
+  GG_CUDA(cudaMemsetAsync(S, 0, 4ull * g->n * k, g->stream));  // rows without in-edges stay 0
+  k_boundary_rows<<<generic_grid(g, std::max<uint64_t>(nblocks, 1)), kGenericThreads, 0, g->stream>>>(
+      si.d_head, si.d_blk, si.d_rows, nblocks, brows.p + 4, brows.p);
+  k_ppr_rows<<<vgrid, kGenericThreads, 0, g->stream>>>(total4, ksh, g->in_off(), g->out_off(), S, T, tbits, damping, XS, 1,
+                                                       iters == 0);
+  g->kernels += 2;
+  for (int32_t it = 0; it < iters; ++it) {
+    if (nblocks) {
+      if (it > 0) {
+        k_zero_rows<<<generic_grid(g, nblocks * k), kGenericThreads, 0, g->stream>>>(brows.p + 4, brows.p, S, k);
+        g->kernels++;
+      }
+      if (k == 64)
+        k_ppr_pull<2><<<pgrid, 256, 0, g->stream>>>(g->in_idx(), si.d_head, si.d_blk, si.d_rows, nblocks, g->m, XS, S,
+                                                    k);
+      else
+        k_ppr_pull<1><<<pgrid, 256, 0, g->stream>>>(g->in_idx(), si.d_head, si.d_blk, si.d_rows, nblocks, g->m, XS, S,
+                                                    k);
+      g->kernels++;
+    }
+    k_ppr_rows<<<vgrid, kGenericThreads, 0, g->stream>>>(total4, ksh, g->in_off(), g->out_off(), S, T, tbits, damping, XS, 0,
+                                                         it == iters - 1);
+    g->kernels++;
   }
+  GG_CUDA(cudaGetLastError());
   return GG_OK;
 }
 
@@ -153,114 +251,79 @@ static int run_ppr_k(gg_graph_s* g, int32_t k, int32_t iters, float damping, con
                      const uint32_t* seeds, float* out, gg_run_stats* st) {
   const uint32_t n = g->n;
   const uint64_t nk = (uint64_t)n * (uint64_t)k;
-  std::vector<uint32_t> brows;
-  boundary_rows(g, brows);
-  float *T = nullptr, *XS = nullptr, *S = nullptr, *Y = nullptr;
-  uint32_t *d_brows = nullptr, *d_seeds = nullptr;
-  auto cleanup = [&]() {
-    cudaFreeAsync(d_seeds, g->stream);
-    cudaFreeAsync(T, g->stream);
-    cudaFreeAsync(XS, g->stream);
-    cudaFreeAsync(S, g->stream);
-    cudaFreeAsync(Y, g->stream);
-    cudaFreeAsync(d_brows, g->stream);
-  };
-  struct Guard {
-    std::function<void()> f;
-    ~Guard() { f(); }
-  } guard{cleanup};
-  GG_CUDA(pool_alloc((void**)&T, 4 * nk, g->stream, g->device));
-  GG_CUDA(pool_alloc((void**)&XS, 4 * nk, g->stream, g->device));
-  GG_CUDA(pool_alloc((void**)&S, 4 * nk, g->stream, g->device));
-  GG_CUDA(pool_alloc((void**)&Y, 4 * nk, g->stream, g->device));
-  GG_CUDA(pool_alloc((void**)&d_brows, 4 * (brows.size() + 1), g->stream, g->device));
-  if (!brows.empty())
-    GG_CUDA(cudaMemcpyAsync(d_brows, brows.data(), 4 * brows.size(), cudaMemcpyHostToDevice, g->stream));
+  DevBuf<float> Tb, XSb, Sb, Yb;
+  DevBuf<uint32_t> seedb, tbitb;
+  GG_TRY(Tb.alloc(g, nk));
+  GG_TRY(XSb.alloc(g, nk));
+  GG_TRY(Sb.alloc(g, nk));
+  float *T = Tb.p, *XS = XSb.p, *S = Sb.p;
   g->kernels = 0;
-  struct EvHold {
-    cudaEvent_t a = nullptr, b = nullptr;
-    ~EvHold() {
-      if (a) cudaEventDestroy(a);
-      if (b) cudaEventDestroy(b);
-    }
-  } ev;
-  cudaEventCreate(&ev.a);
-  cudaEventCreate(&ev.b);
-  cudaEvent_t ea = ev.a, eb = ev.b;
   // inputs are uploaded before the timed region (a renumbered graph's teleport
-  // rows go through Y, which is written only later)
+  // rows go through S, which is written only later)
+  std::vector<uint32_t> dev_seeds;
   if (tele_host) {
-    GG_CUDA(cudaMemcpyAsync(g->relabeled ? Y : T, tele_host, 4 * nk, cudaMemcpyHostToDevice, g->stream));
-    cudaEventRecord(ea, g->stream);
-    if (g->relabeled) GG_TRY(device_order<float>(g, Y, (uint32_t)k, T));
+    GG_CUDA(cudaMemcpyAsync(g->relabeled ? S : T, tele_host, 4 * nk, cudaMemcpyHostToDevice, g->stream));
   } else {
-    std::vector<uint32_t> dev_seeds(seeds, seeds + k);
+    dev_seeds.assign(seeds, seeds + k);
     for (auto& v : dev_seeds) v = g->device_id(v);
-    GG_CUDA(pool_alloc((void**)&d_seeds, 4 * k, g->stream, g->device));
-    GG_CUDA(cudaMemcpyAsync(d_seeds, dev_seeds.data(), 4 * k, cudaMemcpyHostToDevice, g->stream));
-    GG_CUDA(cudaStreamSynchronize(g->stream));  // dev_seeds leaves scope
-    cudaEventRecord(ea, g->stream);
-    GG_CUDA(cudaMemsetAsync(T, 0, 4 * nk, g->stream));
-    k_ppr_onehot<<<1, 64, 0, g->stream>>>(d_seeds, (uint32_t)k, T);
-    g->kernels++;
+    GG_TRY(seedb.alloc(g, k));
+    GG_CUDA(cudaMemcpyAsync(seedb.p, dev_seeds.data(), 4 * k, cudaMemcpyHostToDevice, g->stream));
   }
-  const int grid = generic_grid(g, nk);
-  k_ppr_init<<<grid, kGenericThreads, 0, g->stream>>>(n, (uint32_t)k, T, g->out_off(), XS);
-  g->kernels++;
-  const uint64_t nblocks = (g->m + kSegBlock - 1) / kSegBlock;
-  const SegIndex& si = g->seg[g->transposed ? 1 : 0];
-  const int pgrid = (int)std::min<uint64_t>((nblocks + 7) / 8, (uint64_t)g->num_sms * 16);
-  gg_frontier_s* all = nullptr;
-  if (k == 1) GG_TRY(gg_frontier_all(g, &all));
-  struct AllGuard {
-    gg_frontier_s* f;
-    ~AllGuard() { frontier_free(f); }
-  } all_guard{all};
-  for (int32_t it = 0; it < iters && k == 1; ++it) {
+  EventTimer tm(g->stream);
+  if (tele_host && g->relabeled) GG_TRY(device_order<float>(g, S, (uint32_t)k, T));
+  const float* y = nullptr;
+  if (k > 1) {
+    GG_TRY(tbitb.alloc(g, g->words()));
+    GG_CUDA(cudaMemsetAsync(tbitb.p, 0, 4ull * g->words(), g->stream));
+    if (tele_host) {
+      k_ppr_tbits<<<generic_grid(g, 32ull * n), kGenericThreads, 0, g->stream>>>(n, (uint32_t)k, T, tbitb.p);
+      g->kernels++;
+    } else {
+      k_ppr_seed_rows<<<((uint32_t)k * 32 + 255) / 256, 256, 0, g->stream>>>(seedb.p, (uint32_t)k, T, tbitb.p);
+      k_ppr_onehot<<<1, 64, 0, g->stream>>>(seedb.p, (uint32_t)k, T);
+      g->kernels += 2;
+    }
+    GG_TRY(ppr_columns(g, (uint32_t)k, iters, damping, T, tbitb.p, XS, S));
+    y = XS;
+  } else {
     // one column: the engine's scalar dense pull (edgeMap with every source active)
-    GG_CUDA(cudaMemsetAsync(S, 0, 4 * nk, g->stream));
-    PrPosF f;
-    f.contrib = XS;
-    f.acc_out = S;
-    gg_frontier_s* o = nullptr;
-    GG_TRY(edge_map(g, all, f, (int64_t)g->m / 20, GG_EM_FORCE_CSC | GG_EM_FORCE_COO, &o));
-    frontier_free(o);
-    k_ppr_vertex<<<grid, kGenericThreads, 0, g->stream>>>(n, 1u, g->in_off(), g->out_off(), S, T, damping, Y, XS,
-                                                         it == iters - 1);
-    g->kernels++;
-  }
-  for (int32_t it = 0; it < iters && k > 1; ++it) {
-    if (!brows.empty()) {
-      k_zero_rows<<<generic_grid(g, (uint64_t)brows.size() * k), kGenericThreads, 0, g->stream>>>(
-          d_brows, (uint32_t)brows.size(), S, (uint32_t)k);
+    GG_TRY(Yb.alloc(g, nk));
+    if (!tele_host) {
+      GG_CUDA(cudaMemsetAsync(T, 0, 4 * nk, g->stream));
+      k_ppr_onehot<<<1, 64, 0, g->stream>>>(seedb.p, 1u, T);
       g->kernels++;
     }
-    if (nblocks) {
-      if (k == 64)
-        k_ppr_pull<2><<<std::max(pgrid, 1), 256, 0, g->stream>>>(g->in_idx(), si.d_head, si.d_blk, si.d_rows,
-                                                                  nblocks, g->m, XS, S, (uint32_t)k);
-      else
-        k_ppr_pull<1><<<std::max(pgrid, 1), 256, 0, g->stream>>>(g->in_idx(), si.d_head, si.d_blk, si.d_rows,
-                                                                  nblocks, g->m, XS, S, (uint32_t)k);
+    const int grid = generic_grid(g, nk);
+    k_ppr_init<<<grid, kGenericThreads, 0, g->stream>>>(n, 1u, T, g->out_off(), XS);
+    g->kernels++;
+    gg_frontier_s* all = nullptr;
+    GG_TRY(gg_frontier_all(g, &all));
+    struct AllGuard {
+      gg_frontier_s* f;
+      ~AllGuard() { frontier_free(f); }
+    } all_guard{all};
+    for (int32_t it = 0; it < iters; ++it) {
+      GG_CUDA(cudaMemsetAsync(S, 0, 4 * nk, g->stream));
+      PrPosF f;
+      f.contrib = XS;
+      f.acc_out = S;
+      gg_frontier_s* o = nullptr;
+      GG_TRY(edge_map(g, all, f, (int64_t)g->m / 20, GG_EM_FORCE_CSC | GG_EM_FORCE_COO, &o));
+      frontier_free(o);
+      k_ppr_vertex<<<grid, kGenericThreads, 0, g->stream>>>(n, 1u, g->in_off(), g->out_off(), S, T, damping, Yb.p, XS,
+                                                           it == iters - 1);
       g->kernels++;
     }
-    k_ppr_vertex<<<grid, kGenericThreads, 0, g->stream>>>(n, (uint32_t)k, g->in_off(), g->out_off(), S, T, damping,
-                                                         Y, XS, it == iters - 1);
-    g->kernels++;
+    y = iters ? Yb.p : T;
   }
-  if (iters == 0) GG_CUDA(cudaMemcpyAsync(Y, T, 4 * nk, cudaMemcpyDeviceToDevice, g->stream));
   DevBuf<float> ty;
-  const float* res = Y;
-  GG_TRY(given_order<float>(g, Y, (uint32_t)k, ty, &res));
+  const float* res = y;
+  GG_TRY(given_order<float>(g, y, (uint32_t)k, ty, &res));
   GG_CUDA(cudaGetLastError());
-  cudaEventRecord(eb, g->stream);
-  GG_CUDA(cudaEventSynchronize(eb));
-  float ms = 0;
-  cudaEventElapsedTime(&ms, ea, eb);
-  if (out) {
-    GG_CUDA(cudaMemcpyAsync(out, res, 4 * nk, cudaMemcpyDeviceToHost, g->stream));
-    GG_CUDA(cudaStreamSynchronize(g->stream));
-  }
+  tm.mark();
+  if (out) GG_CUDA(cudaMemcpyAsync(out, res, 4 * nk, cudaMemcpyDeviceToHost, g->stream));
+  GG_CUDA(cudaStreamSynchronize(g->stream));
+  const double ms = tm.elapsed();
   if (st) {
     st->ms = ms;
     st->rounds = iters;
