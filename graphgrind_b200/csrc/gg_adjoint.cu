@@ -47,7 +47,6 @@ static bool wpr_live(const gg_wpr_s* w) {
 // Sums into S: rows inside a block are stored, rows split across blocks added.
 struct SumInto {
   using T = float;
-  static constexpr bool kNeedsIdx = true;
   float* S;
   __device__ static T identity() { return 0.f; }
   __device__ static T combine(T a, T b) { return a + b; }
@@ -60,30 +59,43 @@ struct SumInto {
 };
 
 struct OpFwd : SumInto {  // a_e x[u] over in-edges
+  static constexpr bool kNeedsIdx = true, kNeedsRow = false;
   const float* a;
   const float* x;
-  __device__ float val(uint64_t e, uint32_t y, uint32_t) const { return __ldg(a + e) * __ldg(x + y); }
+  using In = float2;
+  __device__ In load(uint64_t e, uint32_t y, uint32_t) const { return make_float2(ld_stream_f32(a + e), __ldg(x + y)); }
+  __device__ float val(In in, uint64_t) const { return in.x * in.y; }
 };
 struct OpBwd : SumInto {  // a_e lambda[v] over out-edges; dL/da_e += d lambda[v] x_t[u]
+  static constexpr bool kNeedsIdx = true, kNeedsRow = true;
   const float* a;
   const float* lam;
   const float* x;
   float* ga;
   float d;
-  __device__ float val(uint64_t e, uint32_t y, uint32_t row) const {
-    const float l = __ldg(lam + y);
-    ga[e] += d * l * __ldg(x + row);
-    return __ldg(a + e) * l;
+  using In = float4;
+  __device__ In load(uint64_t e, uint32_t y, uint32_t row) const {
+    return make_float4(ld_stream_f32(a + e), __ldg(lam + y), __ldg(x + row), ga[e]);
+  }
+  __device__ float val(In in, uint64_t e) const {
+    ga[e] = in.w + d * in.y * in.z;
+    return in.x * in.y;
   }
 };
 struct OpW : SumInto {  // sum of out-edge weights
+  static constexpr bool kNeedsIdx = false, kNeedsRow = false;
   const float* w;
-  __device__ float val(uint64_t e, uint32_t, uint32_t) const { return __ldg(w + e); }
+  using In = float;
+  __device__ In load(uint64_t e, uint32_t, uint32_t) const { return __ldg(w + e); }
+  __device__ float val(In in, uint64_t) const { return in; }
 };
 struct OpNormBack : SumInto {  // sum of dL/da_e * a_e over out-edges
+  static constexpr bool kNeedsIdx = false, kNeedsRow = false;
   const float* ga;
   const float* a;
-  __device__ float val(uint64_t e, uint32_t, uint32_t) const { return __ldg(ga + e) * __ldg(a + e); }
+  using In = float2;
+  __device__ In load(uint64_t e, uint32_t, uint32_t) const { return make_float2(__ldg(ga + e), __ldg(a + e)); }
+  __device__ float val(In in, uint64_t) const { return in.x * in.y; }
 };
 
 template <class Op>

@@ -23,18 +23,20 @@ __device__ __forceinline__ void atomic_mul(float* a, float b) {
 
 struct BpOp {
   using T = float2;
-  static constexpr bool kNeedsIdx = false;
+  static constexpr bool kNeedsIdx = false, kNeedsRow = true;
   const float2* vp;   // [n] vertex potentials
   const float4* ep;   // [m] edge potentials, (i, k) at component 2 i + k
   const float2* cur;  // [n] products of the previous iteration
   float2* next;       // [n] products of this iteration (reset to 1)
   __device__ static T identity() { return make_float2(1.f, 1.f); }
   __device__ static T combine(T a, T b) { return make_float2(a.x * b.x, a.y * b.y); }
-  __device__ T val(uint64_t e, uint32_t, uint32_t row) const {
+  using In = float2;
+  __device__ In load(uint64_t e, uint32_t, uint32_t row) const {
     const float2 p = __ldg(vp + row), c = __ldg(cur + row);
     const float4 w = __ldg(ep + e);
     return make_float2(p.x * w.x * c.x + p.y * w.y * c.y, p.x * w.z * c.x + p.y * w.w * c.y);
   }
+  __device__ T val(In in, uint64_t) const { return in; }
   __device__ void flush(uint32_t row, T v, bool complete) const {
     if (complete) {
       next[row] = v;

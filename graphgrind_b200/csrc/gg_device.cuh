@@ -53,6 +53,17 @@ __device__ __forceinline__ uint4 ld_stream_v4(const void* ptr, uint64_t pol) {
       : "l"(ptr), "l"(pol));
   return r;
 }
+// 4-byte read-only load that bypasses L1 (streamed data).
+__device__ __forceinline__ uint32_t ld_stream_u32(const uint32_t* ptr) {
+  uint32_t r;
+  asm("ld.global.nc.L1::no_allocate.u32 %0, [%1];" : "=r"(r) : "l"(ptr));
+  return r;
+}
+__device__ __forceinline__ float ld_stream_f32(const float* ptr) {
+  float r;
+  asm("ld.global.nc.L1::no_allocate.f32 %0, [%1];" : "=f"(r) : "l"(ptr));
+  return r;
+}
 // 4-byte read-only gather kept in L1 and L2 ahead of streamed lines.
 __device__ __forceinline__ float ld_keep_f32(const float* ptr, uint64_t pol) {
   float r;
