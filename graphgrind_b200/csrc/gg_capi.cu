@@ -863,6 +863,7 @@ __global__ void k_round_check(RoundLoopCtl* c, unsigned long long* stats, unsign
 static bool round_takes_coo(const gg_graph_s* g, const gg_frontier_s* f) {
   const int64_t fm = (int64_t)f->dm, tot = (int64_t)f->out_edges, m = (int64_t)g->m;
   if (f->bit || tot == 0 || !g->has_coo || fm + tot <= app_threshold(g)) return false;
+  if (dense_takes_coo(g)) return true;
   const bool ref_rule = g->dense_policy == 0 || g->transposed;
   return ref_rule ? fm + tot > m / 2 : g->dense_policy == 2;
 }
@@ -1033,7 +1034,7 @@ static int round_loop_run(gg_graph_s* g, RoundLoop* L, FrontierHold& F, uint32_t
   c.threshold = app_threshold(g);
   c.dense_threshold = (long long)g->m / 2;
   c.max_rounds = max_rounds;
-  c.coo_always = (g->dense_policy == 0 || g->transposed) ? 0u : 1u;
+  c.coo_always = dense_takes_coo(g) || !(g->dense_policy == 0 || g->transposed) ? 1u : 0u;
   c.use_l1 = l1 ? 1u : 0u;
   c.eps = eps;
   GG_TRY(write_small(g, L->d_ctl, c));

@@ -555,6 +555,18 @@ int push_bits_launch(gg_graph_s* g, gg_frontier_s* in, gg_frontier_s* out, const
   return GG_OK;
 }
 
+// Dense steps that edgeMap's rule sends to the CSC pull (frontiers between the
+// direction threshold and m/2) run on the partitioned COO, where the graph has
+// one for the default kernel: both apply the same gathers and commits to the
+// same edges, and the COO's destination tiles with Hilbert-ordered sources
+// keep more of the gathers in L1 (a step over all edges with half the vertices
+// active, COO / CSC: R-MAT-20 92 / 275 us, Erdos-Renyi with 24M edges 154 /
+// 394, R-MAT-22 renumbered 230 / 1390).  Not for a transposed graph, whose COO
+// is not transposed, nor under a dense policy or flag that names the kernel.
+inline bool dense_takes_coo(const gg_graph_s* g) {
+  return g->dense_policy == 0 && !g->transposed && g->has_coo && !g->coo_by_source && g->coo_kernel >= 6;
+}
+
 // Internal edge_map flag (beside the GG_EM_* bits of the C ABI, which
 // gg_edge_map passes on alone): with GG_EM_NO_OUTPUT, the caller waits for the
 // stream itself, so the call need not.
@@ -606,6 +618,9 @@ int edge_map(gg_graph_s* g, gg_frontier_s* in, const F& f, int64_t threshold, ui
     if (flags & GG_EM_FORCE_CSC) coo = false;
     if ((flags & GG_EM_FORCE_COO) && g->has_coo) coo = true;
     const bool early = !coo && F::kEarlyExit;
+    // the kernel; g->last.kind and the output stay those of the rule.  The
+    // vertex step at the commits (PrFinishF) belongs to the rule's COO steps.
+    const bool coo_pull = coo || (!early && !finishes<F>::value && !(flags & GG_EM_FORCE_CSC) && dense_takes_coo(g));
     // a dense step of an early-exit functor from few frontier vertices (a
     // hub level): push the frontier's out-edges into the output bitmap
     // instead of walking every unvisited in-list
@@ -628,7 +643,8 @@ int edge_map(gg_graph_s* g, gg_frontier_s* in, const F& f, int64_t threshold, ui
       else if (early)
         rc = hw ? pull_early_launch<F, true>(g, in, o, f) : pull_early_launch<F, false>(g, in, o, f);
       else
-        rc = hw ? pull_launch<F, true>(g, in, o, f, coo, no_out) : pull_launch<F, false>(g, in, o, f, coo, no_out);
+        rc = hw ? pull_launch<F, true>(g, in, o, f, coo_pull, no_out)
+                : pull_launch<F, false>(g, in, o, f, coo_pull, no_out);
       if (g->profiling) cudaEventRecord(g->prof_ev[1], g->stream);
     }
     // an output nobody reads from a pull without waits (the direct-load COO
@@ -652,7 +668,8 @@ int edge_map(gg_graph_s* g, gg_frontier_s* in, const F& f, int64_t threshold, ui
       o->dm = g->ws.h_stats[0];
       o->out_edges = g->ws.h_stats[1];
       g->last.kind = coo ? 3 : 2;
-      prof_end(push_bits ? 0 : (early ? 3 : (coo ? 2 : 1)), push_bits ? (uint64_t)tot : (coo ? g->coo_len : g->m));
+      prof_end(push_bits ? 0 : (early ? 3 : (coo_pull ? 2 : 1)),
+               push_bits ? (uint64_t)tot : (coo_pull ? g->coo_len : g->m));
     }
   } else {
     if (!in->has_sparse) rc = frontier_to_sparse(in);

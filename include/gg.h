@@ -321,7 +321,9 @@ int gg_graph_set_profiling(gg_graph_t g, int32_t enable);
 /* Copies the accumulated profile and resets it. */
 int gg_graph_get_profile(gg_graph_t g, gg_profile* out);
 /* Dense-branch kernel policy: 0 = the reference's rule (COO above m/2 when
- * the COO exists, else CSC), 1 = always CSC pull, 2 = always COO pull. */
+ * the COO exists, else CSC; gg_edge_map_stats.kind reports it, while the pull
+ * itself runs on the COO below m/2 too where that gives the same result
+ * faster), 1 = always CSC pull, 2 = always COO pull. */
 int gg_graph_set_dense_policy(gg_graph_t g, int32_t policy);
 /* Engine tuning knobs (all keep edgeMap's results; they pick kernels):
  *   GG_TUNE_DENSE_POLICY  as gg_graph_set_dense_policy
