@@ -73,7 +73,7 @@ constexpr int kMaxCooTileVertices = 16384;  // COO tiles (16-bit destination off
 constexpr uint32_t kPad = 0xffffffffu;                      // COO padding source id
 
 constexpr int kPushThreads = 256;
-constexpr int kPushEdgesPerCta = 4096;
+constexpr int kPushEdgesPerCta = 4096;  // of k_push_bits
 constexpr int kScanThreads = 256;
 constexpr int kScanItems = 8;
 constexpr int kScanTile = kScanThreads * kScanItems;        // 2048 queue entries per block
@@ -1631,6 +1631,35 @@ static __global__ void __launch_bounds__(kScanThreads) k_scan_write(const uint32
   }
 }
 
+// The three passes as one CTA of 1024 threads for queues of at most
+// kScanOne entries, which also clears the step's counters (stats[8]).
+constexpr uint32_t kScanOne = 1024 * kScanItems;
+static __global__ void __launch_bounds__(1024) k_scan_one(const uint32_t* q, uint32_t k, const uint32_t* off,
+                                                          uint32_t* offs, unsigned long long* stats) {
+  __shared__ uint32_t s_warp[32];
+  const uint32_t base = threadIdx.x * kScanItems;
+  uint32_t d[kScanItems];
+  uint32_t t = 0;
+#pragma unroll
+  for (int i = 0; i < kScanItems; ++i) {
+    d[i] = 0;
+    if (base + i < k) {
+      const uint32_t v = q[base + i];
+      d[i] = off[v + 1] - off[v];
+    }
+    t += d[i];
+  }
+  uint32_t tot;
+  uint32_t run = block_excl_scan(t, s_warp, &tot);
+#pragma unroll
+  for (int i = 0; i < kScanItems; ++i) {
+    if (base + i < k) offs[base + i] = run;
+    run += d[i];
+  }
+  if (threadIdx.x == 0) offs[k] = tot;
+  if (threadIdx.x < 8) stats[threadIdx.x] = threadIdx.x == 5 ? tot : 0ull;
+}
+
 struct PushParams {
   const uint32_t* q;        // frontier queue
   uint32_t k;               // queue length
@@ -1705,67 +1734,115 @@ __global__ void __launch_bounds__(kPushThreads) k_push_bits(const PushParams p, 
   }
 }
 
+// Sparse push.  A sparse step is bound by its chain of dependent loads, so the
+// edges go to the CTAs one window of 256 at a time as long as the grid has
+// CTAs (with 4096 edges per CTA, a step of 100K edges ran 16 windows deep on 25
+// CTAs: 29 us, now 8), a CTA finds its first queue slot by 256-way search
+// rounds, stages the slots of its window in shared memory, and appends with
+// one atomic.
 template <class F, bool HW>
 __global__ void __launch_bounds__(kPushThreads) k_push(const PushParams p, const F f) {
-  __shared__ uint32_t s_q[2];
+  __shared__ uint32_t s_off[kPushThreads], s_q[kPushThreads], s_beg[kPushThreads];
+  __shared__ uint32_t s_cnt[kPushThreads / 32];
+  __shared__ uint32_t s_base;
+  __shared__ unsigned long long s_deg[kPushThreads / 32];
   const uint64_t E = *p.total;
-  const int lane = threadIdx.x & 31;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   unsigned long long my_deg = 0;
-  for (uint64_t c = blockIdx.x; c * kPushEdgesPerCta < E; c += gridDim.x) {
-    const uint32_t e_lo = (uint32_t)(c * kPushEdgesPerCta);
-    const uint64_t e_end = (uint64_t)e_lo + kPushEdgesPerCta;
-    const uint32_t e_hi = (uint32_t)(E < e_end ? E : e_end);
-    if (threadIdx.x < 2) {
-      const uint32_t key = threadIdx.x == 0 ? e_lo : e_hi - 1;
-      uint32_t lo = 0, hi = p.k;  // largest i with offs[i] <= key
+  const uint64_t windows = (E + kPushThreads - 1) / kPushThreads;
+  const uint64_t per = (windows + gridDim.x - 1) / gridDim.x;
+  const uint64_t w1 = windows < (blockIdx.x + 1) * per ? windows : (blockIdx.x + 1) * per;
+  uint32_t scur = 0;
+  for (uint64_t w = blockIdx.x * per; w < w1; ++w) {
+    const uint32_t base = (uint32_t)(w * kPushThreads);
+    const uint32_t last = (uint32_t)(E < (w + 1) * kPushThreads ? E - 1 : (w + 1) * kPushThreads - 1);
+    // the slot that holds the window's first edge: the last one whose offset
+    // is at most that (a queue of one stage is staged whole)
+    if (p.k > kPushThreads) {
+      uint32_t lo = scur, hi = p.k;
       while (hi - lo > 1) {
-        const uint32_t mid = (lo + hi) >> 1;
-        if (p.offs[mid] <= key) lo = mid; else hi = mid;
+        const uint32_t step = (hi - lo + kPushThreads - 1) / kPushThreads;
+        const uint64_t probe = lo + (uint64_t)tid * step;
+        const int cnt = __syncthreads_count(probe < hi && p.offs[probe] <= base);
+        lo += (uint32_t)(cnt - 1) * step;
+        hi = hi - lo < step ? hi : lo + step;
       }
-      s_q[threadIdx.x] = lo;
+      scur = lo;
     }
-    __syncthreads();
-    const uint32_t qlo = s_q[0], qhi = s_q[1];
-    const uint32_t iters = (e_hi - e_lo + kPushThreads - 1) / kPushThreads;
-    for (uint32_t it = 0; it < iters; ++it) {
-      const uint32_t e = e_lo + it * kPushThreads + threadIdx.x;
-      bool take = false;
-      uint32_t d = 0;
-      if (e < e_hi) {
-        uint32_t lo = qlo, hi = qhi + 1;
+    const uint64_t sl = (uint64_t)scur + tid;
+    const uint32_t o = sl < p.k ? p.offs[sl] : 0xffffffffu;
+    const bool mine = sl < p.k && o <= last;
+    s_off[tid] = o;
+    if (mine) {
+      const uint32_t v = p.q[sl];
+      s_q[tid] = v;
+      s_beg[tid] = p.off[v];
+    }
+    const int ns = __syncthreads_count(mine);
+    // vertices without out-edges take slots but no edges, so the window may
+    // reach past the staged slots; its threads then search the queue itself
+    const bool past = ns == kPushThreads && (uint64_t)scur + ns < p.k && p.offs[scur + ns] <= last;
+    const uint32_t e = base + tid;
+    bool take = false;
+    uint32_t d = 0;
+    if (e <= last) {
+      uint32_t s, ei;
+      if (!past) {
+        int lo = 0, hi = ns;
         while (hi - lo > 1) {
-          const uint32_t mid = (lo + hi) >> 1;
+          const int mid = (lo + hi) >> 1;
+          if (s_off[mid] <= e) lo = mid; else hi = mid;
+        }
+        s = s_q[lo];
+        ei = s_beg[lo] + (e - s_off[lo]);
+      } else {
+        uint32_t lo = scur, hi = p.k;
+        while (hi - lo > 1) {
+          const uint32_t mid = lo + (hi - lo) / 2;
           if (p.offs[mid] <= e) lo = mid; else hi = mid;
         }
-        const uint32_t s = p.q[lo];
-        const uint32_t ei = p.off[s] + (e - p.offs[lo]);
-        d = p.idx[ei];
-        const uint32_t w = HW ? p.wts[ei] : 1u;
-        if (f.cond(d) && f.update_atomic(s, d, w)) {
-          const uint32_t bit = 1u << (d & 31);
-          take = !(atomicOr(p.dedup + (d >> 5), bit) & bit);
-        }
+        s = p.q[lo];
+        ei = p.off[s] + (e - p.offs[lo]);
       }
-      const uint32_t ball = __ballot_sync(0xffffffffu, take);
-      if (ball) {
-        uint32_t base = 0;
-        if (lane == 0) base = (uint32_t)atomicAdd(p.stats + 2, (unsigned long long)__popc(ball));
-        base = __shfl_sync(0xffffffffu, base, 0);
-        if (take) {
-          p.out_q[base + __popc(ball & ((1u << lane) - 1u))] = d;
-          my_deg += p.deg_off[d + 1] - p.deg_off[d];
-        }
+      d = p.idx[ei];
+      const uint32_t wt = HW ? p.wts[ei] : 1u;
+      if (f.cond(d) && f.update_atomic(s, d, wt)) {
+        const uint32_t bit = 1u << (d & 31);
+        take = !(atomicOr(p.dedup + (d >> 5), bit) & bit);
       }
     }
+    const uint32_t ball = __ballot_sync(0xffffffffu, take);
+    if (lane == 0) s_cnt[warp] = __popc(ball);
     __syncthreads();
+    uint32_t before = 0, all = 0;
+#pragma unroll
+    for (int i = 0; i < kPushThreads / 32; ++i) {
+      if (i < warp) before += s_cnt[i];
+      all += s_cnt[i];
+    }
+    if (tid == 0 && all) s_base = (uint32_t)atomicAdd(p.stats + 2, (unsigned long long)all);
+    __syncthreads();
+    if (take) {
+      p.out_q[s_base + before + __popc(ball & ((1u << lane) - 1u))] = d;
+      my_deg += p.deg_off[d + 1] - p.deg_off[d];
+    }
   }
   my_deg = warp_sum(my_deg);
-  if (lane == 0 && my_deg) atomicAdd(p.stats + 1, my_deg);
+  if (lane == 0) s_deg[warp] = my_deg;
+  __syncthreads();
+  if (tid == 0) {
+    unsigned long long t = 0;
+    for (int i = 0; i < kPushThreads / 32; ++i) t += s_deg[i];
+    if (t) atomicAdd(p.stats + 1, t);
+  }
 }
 
-// zero the dedup words touched by a queue
-static __global__ void k_clear_dedup(const uint32_t* q, const unsigned long long* len, uint32_t* dedup) {
-  const uint64_t k = *len;
+// zero the dedup words touched by a queue; with `map`, the step's counters go
+// to the host's mapped block in the same launch
+static __global__ void k_clear_dedup(const uint32_t* q, const unsigned long long* stats, uint32_t* dedup,
+                                     unsigned long long* map = nullptr) {
+  if (map && blockIdx.x == 0 && threadIdx.x < 8) map[threadIdx.x] = stats[threadIdx.x];
+  const uint64_t k = stats[2];
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < k; i += (uint64_t)gridDim.x * blockDim.x)
     dedup[q[i] >> 5] = 0u;
 }

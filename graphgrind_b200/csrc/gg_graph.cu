@@ -194,6 +194,14 @@ int read_stats(gg_graph_s* g) {
   return GG_OK;
 }
 
+int read_stats_end(gg_graph_s* g) {
+  GG_CUDA(cudaStreamSynchronize(g->stream));
+  read_small_end(g, g->ws.h_stats, 8);
+  if (g->ws.h_stats[3])
+    return fail(GG_ERR_TIMEOUT, "device wait budget exhausted (error word %llu)", (unsigned long long)g->ws.h_stats[3]);
+  return GG_OK;
+}
+
 // ------------------------------------------------------------------ tiles
 // Greedy destination tiles over [vbeg, vend): at most tv vertices and about
 // te edges (a single vertex above te gets its own tile); edge-less ranges

@@ -121,7 +121,7 @@ extern "C" int gg_bfs_push_step_noalloc(const uint32_t* out_offsets, const uint3
     gg::k_push<gg::BfsF, false><<<num_sms * 8, gg::kPushThreads, 0, st>>>(p, f);
     GG_CUDA(cudaGetLastError());
     // the output's dedup words back to zero for the next call
-    gg::k_clear_dedup<<<num_sms * 4, 256, 0, st>>>(next_frontier, stats + 2, dedup);
+    gg::k_clear_dedup<<<num_sms * 4, 256, 0, st>>>(next_frontier, stats, dedup);
     GG_CUDA(cudaGetLastError());
   }
   // next_counts[0] = output frontier size, next_counts[1] = its out-degree sum

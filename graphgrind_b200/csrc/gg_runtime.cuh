@@ -273,6 +273,7 @@ int reset_stats(gg_graph_s* g);
 void pr_loop_free(gg_graph_s* g);  // releases the captured PageRank loop and its buffers
 void round_loops_free(gg_graph_s* g);  // the same for the BellmanFord / Components round loops
 int read_stats(gg_graph_s* g);  // blocks; checks the device error word
+int read_stats_end(gg_graph_s* g);  // the same for counters a kernel has put into the mapped block
 
 // -------------------------------------------------------------- edgeMap
 // graphgrind/ligra-numa.h:919-1019
@@ -482,20 +483,29 @@ int pull_early_launch(gg_graph_s* g, gg_frontier_s* in, gg_frontier_s* out, cons
   return GG_OK;
 }
 
+// One sparse step: clears the counters, and leaves them in the mapped block
+// (read_stats_end) once the stream has passed.
 template <class F, bool HW>
 int push_launch(gg_graph_s* g, gg_frontier_s* in, gg_frontier_s* out, const F& f) {
   const uint32_t k = (uint32_t)in->dm;
-  const uint32_t nb = (k + kScanTile - 1) / kScanTile;
   Workspace& ws = g->ws;
-  if (nb > ws.bsum_cap) {
-    if (ws.d_bsum) cudaFree(ws.d_bsum);
-    GG_CUDA(cudaMalloc(&ws.d_bsum, sizeof(uint32_t) * (nb + 32)));
-    ws.bsum_cap = nb;
-  }
   const uint32_t* off = g->out_off();
-  k_scan_sums<<<nb, kScanThreads, 0, g->stream>>>(in->d_queue, k, off, ws.d_bsum);
-  k_scan_blocks<<<1, 1024, 0, g->stream>>>(ws.d_bsum, nb, ws.d_stats + 5);
-  k_scan_write<<<nb, kScanThreads, 0, g->stream>>>(in->d_queue, k, off, ws.d_bsum, ws.d_scan);
+  if (k <= kScanOne) {
+    k_scan_one<<<1, 1024, 0, g->stream>>>(in->d_queue, k, off, ws.d_scan, ws.d_stats);
+    g->kernels++;
+  } else {
+    const uint32_t nb = (k + kScanTile - 1) / kScanTile;
+    if (nb > ws.bsum_cap) {
+      if (ws.d_bsum) cudaFree(ws.d_bsum);
+      GG_CUDA(cudaMalloc(&ws.d_bsum, sizeof(uint32_t) * (nb + 32)));
+      ws.bsum_cap = nb;
+    }
+    GG_TRY(reset_stats(g));
+    k_scan_sums<<<nb, kScanThreads, 0, g->stream>>>(in->d_queue, k, off, ws.d_bsum);
+    k_scan_blocks<<<1, 1024, 0, g->stream>>>(ws.d_bsum, nb, ws.d_stats + 5);
+    k_scan_write<<<nb, kScanThreads, 0, g->stream>>>(in->d_queue, k, off, ws.d_bsum, ws.d_scan);
+    g->kernels += 3;
+  }
   PushParams p{};
   p.q = in->d_queue;
   p.k = k;
@@ -508,14 +518,14 @@ int push_launch(gg_graph_s* g, gg_frontier_s* in, gg_frontier_s* out, const F& f
   p.dedup = ws.d_dedup;
   p.out_q = out->d_queue;
   p.stats = ws.d_stats;
-  // persistent CTAs: the edge total is read on the device
-  const uint64_t work_ub = std::max<uint64_t>(in->out_edges, 1);
-  const int grid = (int)std::min<uint64_t>((work_ub + kPushEdgesPerCta - 1) / kPushEdgesPerCta + 1,
-                                           (uint64_t)g->num_sms * 8);
-  k_push<F, HW><<<std::max(grid, g->num_sms), kPushThreads, 0, g->stream>>>(p, f);
-  k_clear_dedup<<<g->num_sms, kGenericThreads, 0, g->stream>>>(out->d_queue, ws.d_stats + 2, ws.d_dedup);
+  const int grid = generic_grid(g, std::max<uint64_t>(in->out_edges, 1));
+  static_assert(kGenericThreads == kPushThreads, "a CTA per window of edges");
+  k_push<F, HW><<<grid, kPushThreads, 0, g->stream>>>(p, f);
+  // the output holds at most an entry per edge
+  k_clear_dedup<<<std::min(grid, g->num_sms), kGenericThreads, 0, g->stream>>>(
+      out->d_queue, ws.d_stats, ws.d_dedup, reinterpret_cast<unsigned long long*>(ws.d_map));
   GG_CUDA(cudaGetLastError());
-  g->kernels += 5;
+  g->kernels += 2;
   return GG_OK;
 }
 
@@ -674,19 +684,18 @@ int edge_map(gg_graph_s* g, gg_frontier_s* in, const F& f, int64_t threshold, ui
   } else {
     if (!in->has_sparse) rc = frontier_to_sparse(in);
     if (!rc) rc = frontier_ensure_queue(o);
-    if (!rc) rc = reset_stats(g);
-    if (!rc && in->dm > 0) {
+    if (!rc) {  // tot > 0, so the frontier has members
       prof_begin();
       rc = hw ? push_launch<F, true>(g, in, o, f) : push_launch<F, false>(g, in, o, f);
       if (g->profiling) cudaEventRecord(g->prof_ev[1], g->stream);
     }
-    if (!rc) rc = read_stats(g);
+    if (!rc) rc = read_stats_end(g);
     if (!rc) {
       o->has_sparse = true;
       o->dm = g->ws.h_stats[2];
       o->out_edges = g->ws.h_stats[1];
       g->last.kind = 1;
-      if (in->dm > 0) prof_end(0, g->ws.h_stats[5]);
+      prof_end(0, g->ws.h_stats[5]);
     }
   }
   if (rc) {
