@@ -125,19 +125,92 @@ __global__ void k_pr_epilogue(uint32_t n, int all, const uint32_t* fbits, float*
   block_add_double(acc, l1);
 }
 
-// PageRankDelta round epilogue (app/PageRankDelta.C:158-165): L1 = sum|Delta|,
-// nghSum reset to 0, next round's contrib = Delta/outdeg.
-__global__ void k_prd_epilogue(uint32_t n, const float* delta, float* ngh, const uint32_t* off, float* contrib,
-                               double* l1) {
+// PageRankDelta's vertex work of a round in one pass (app/PageRankDelta.C:
+// 73-105 and 158-165): the vertexFilter over all vertices (PR_Vertex_F, in the
+// first round PR_Vertex_F_FirstRound) into out_bits with its count and
+// out-degree sum, L1 = sum |Delta|, nghSum reset to 0 and the next round's
+// contrib = Delta/outdeg.  It moves 32 bytes per vertex; the counts take one
+// atomic per CTA (a filter with one per warp and a separate epilogue took 18
+// us on R-MAT-20, this FIGURE).
+template <bool FIRST>
+__global__ void __launch_bounds__(256) k_prd_vertex(uint32_t n, float* p, float* delta, float* ngh,
+                                                    const uint32_t* __restrict__ off, float* contrib, uint32_t* out_bits, unsigned long long* stats,
+                                                    double* l1, float damping, float added, float one_over_n,
+                                                    float eps2) {
+  constexpr int U = 2;  // 32-vertex groups in flight per warp
+  __shared__ unsigned long long s_sum[2][8];
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+  unsigned long long cnt = 0, deg = 0;
   double acc = 0;
-  for (uint64_t j = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; j < n; j += (uint64_t)gridDim.x * blockDim.x) {
-    const float dl = delta[j];
-    acc += fabsf(dl);
-    ngh[j] = 0.0f;
-    const uint32_t d = off[j + 1] - off[j];
-    contrib[j] = d ? dl / (float)d : 0.0f;
+  for (uint64_t b0 = (uint64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31u); b0 < n; b0 += U * stride) {
+    float pv[U], nv[U];
+    uint32_t dg[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const uint64_t v = b0 + u * stride + lane;
+      pv[u] = nv[u] = 0.f;
+      dg[u] = 0;
+      if (v < n) {
+        pv[u] = p[v];
+        nv[u] = ngh[v];
+        dg[u] = off[v + 1] - off[v];
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const uint64_t b = b0 + u * stride;
+      if (b >= n) break;  // warp-uniform
+      const uint64_t v = b + lane;
+      bool act = false;
+      if (v < n) {
+        float d, pi;
+        if (FIRST) {
+          d = damping * (pv[u] + nv[u]) + added - pv[u];
+          pi = pv[u] + d;
+          d -= one_over_n;
+        } else {
+          d = nv[u] * damping;
+          pi = pv[u] + d;
+        }
+        p[v] = pi;
+        delta[v] = d;
+        ngh[v] = 0.0f;
+        contrib[v] = dg[u] ? d / (float)dg[u] : 0.0f;
+        acc += fabsf(d);
+        act = fabsf(d) > eps2 * pi;
+        if (act) deg += dg[u];
+      }
+      const uint32_t word = __ballot_sync(0xffffffffu, act);
+      if (lane == 0) {
+        out_bits[b >> 5] = word;
+        cnt += __popc(word);
+      }
+    }
   }
-  block_add_double(acc, l1);
+  deg = warp_sum(deg);
+  if (lane == 0) {
+    s_sum[0][warp] = cnt;
+    s_sum[1][warp] = deg;
+  }
+  block_add_double(acc, l1);  // its block barrier covers s_sum
+  if (threadIdx.x < 2) {
+    unsigned long long t = 0;
+    for (int w = 0; w < 8; ++w) t += s_sum[threadIdx.x][w];
+    if (t) atomicAdd(stats + threadIdx.x, t);
+  }
+}
+
+template <bool FIRST>
+static int prd_vertex(gg_graph_s* g, float* p, float* delta, float* ngh, float* contrib, uint32_t* out_bits,
+                      unsigned long long* stats) {
+  const double n = (double)g->n;
+  k_prd_vertex<FIRST><<<generic_grid(g, g->n), kGenericThreads, 0, g->stream>>>(
+      g->n, p, delta, ngh, g->out_off(), contrib, out_bits, stats, g->ws.d_red, 0.85f, (float)((1 - 0.85) * (1 / n)),
+      (float)(1 / n), 0.01f);
+  GG_CUDA(cudaGetLastError());
+  g->kernels++;
+  return GG_OK;
 }
 
 __global__ void k_invert(uint32_t n, float* a) {
@@ -150,6 +223,21 @@ __global__ void k_bc_final(uint32_t n, float* dep, const float* inv) {
 }
 
 static int read_red(gg_graph_s* g, double* v) { return read_small(g, v, g->ws.d_red); }
+
+// The step's counters (h_stats) and a reduction, with one wait.
+__global__ void k_get_stats_red(unsigned long long* dst, const unsigned long long* stats, const double* red) {
+  if (threadIdx.x < 8) dst[threadIdx.x] = __ldcg(stats + threadIdx.x);
+  if (threadIdx.x == 8) reinterpret_cast<double*>(dst)[8] = __ldcg(red);
+}
+static int read_stats_red(gg_graph_s* g, double* v) {
+  k_get_stats_red<<<1, 32, 0, g->stream>>>(reinterpret_cast<unsigned long long*>(g->ws.d_map), g->ws.d_stats,
+                                           g->ws.d_red);
+  GG_CUDA(cudaGetLastError());
+  g->kernels++;
+  GG_TRY(read_stats_end(g));
+  std::memcpy(v, reinterpret_cast<const unsigned long long*>(g->ws.h_map) + 8, sizeof(double));
+  return GG_OK;
+}
 
 static void fill_stats(gg_run_stats* st, double ms, int rounds, uint64_t trav, int kernels) {
   if (!st) return;
@@ -820,9 +908,10 @@ void round_loops_free(gg_graph_s* g) {
 }
 
 // fstats: where the round's next frontier was counted (PageRankDelta's
-// vertexFilter), else the pull's own counters in stats; red: the round's L1.
+// vertexFilter), else the pull's own counters in stats; red: the round's L1,
+// cleared for the next.
 __global__ void k_round_check(RoundLoopCtl* c, unsigned long long* stats, unsigned long long* fstats,
-                              const double* red, cudaGraphConditionalHandle h_loop,
+                              double* red, cudaGraphConditionalHandle h_loop,
                               cudaGraphConditionalHandle h_odd, int set_odd, uint32_t* clear_bits,
                               uint32_t clear_words) {
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < clear_words;
@@ -836,7 +925,10 @@ __global__ void k_round_check(RoundLoopCtl* c, unsigned long long* stats, unsign
   c->count = count;
   c->dm = dm;
   c->out_edges = oe;
-  if (c->use_l1) c->l1 = red[0];
+  if (c->use_l1) {
+    c->l1 = red[0];
+    red[0] = 0;
+  }
   uint32_t reason = 0;
   if (err) {
     c->err = err;
@@ -909,16 +1001,7 @@ static int round_launches(gg_graph_s* g, RoundLoop* L, int app, uint32_t* in_bit
   f.contrib = contrib;
   f.acc_out = ngh;
   GG_TRY((pull_launch<PrF, false>(g, &in, &out, f, true)));
-  const VPrd vf{p, delta, ngh, 0.85f, 0.01f};
-  k_vertex_filter<VPrd, true><<<generic_grid(g, g->n), kGenericThreads, 0, g->stream>>>(
-      g->n, nullptr, out_bits, g->out_off(), L->d_fstats, vf);
-  GG_CUDA(cudaGetLastError());
-  GG_CUDA(cudaMemsetAsync(g->ws.d_red, 0, sizeof(double), g->stream));
-  k_prd_epilogue<<<generic_grid(g, g->n), kGenericThreads, 0, g->stream>>>(g->n, delta, ngh, g->out_off(), contrib,
-                                                                           g->ws.d_red);
-  GG_CUDA(cudaGetLastError());
-  g->kernels += 2;
-  return GG_OK;
+  return prd_vertex<false>(g, p, delta, ngh, contrib, out_bits, L->d_fstats);
 }
 
 static int round_loop_capture(gg_graph_s* g, RoundLoop* L, int app) {
@@ -1029,6 +1112,7 @@ static int round_loop_run(gg_graph_s* g, RoundLoop* L, FrontierHold& F, uint32_t
   GG_CUDA(cudaMemcpyAsync(L->bits[0], in->d_bits, bb, cudaMemcpyDeviceToDevice, g->stream));
   GG_CUDA(cudaMemsetAsync(L->bits[1], 0, bb, g->stream));
   GG_TRY(reset_stats(g));
+  if (l1) GG_CUDA(cudaMemsetAsync(g->ws.d_red, 0, sizeof(double), g->stream));
   RoundLoopCtl& c = *L->h_ctl;
   c = RoundLoopCtl{};
   c.threshold = app_threshold(g);
@@ -1318,19 +1402,15 @@ static int run_pagerank_delta(gg_graph_s* g, float* ranks, gg_run_stats* st) {
     ngh = nghb.p;
     contrib = contribb.p;
   }
-  const float damping = 0.85f, eps2 = 0.01f;  // the round graph's vertexFilter uses the same constants
   const double eps = 0.0000001;
-  const float one_over_n = (float)(1 / (double)n);
-  const float added = (float)((1 - 0.85) * (1 / (double)n));
   EventTimer tm(g->stream);
   GG_TRY(fill<float>(g, p, n, 0.0f));
-  GG_TRY(fill<float>(g, delta, n, one_over_n));
+  GG_TRY(fill<float>(g, delta, n, (float)(1 / (double)n)));
   GG_TRY(fill<float>(g, ngh, n, 0.0f));
   k_div_outdeg<<<generic_grid(g, n), kGenericThreads, 0, g->stream>>>(n, delta, g->out_off(), contrib);
   g->kernels++;
-  FrontierHold F, All;
+  FrontierHold F;
   GG_TRY(gg_frontier_all(g, &F.f));
-  GG_TRY(gg_frontier_all(g, &All.f));
   int64_t round = 0;
   uint64_t trav = 0;
   for (;;) {
@@ -1348,23 +1428,18 @@ static int run_pagerank_delta(gg_graph_s* g, float* ranks, gg_run_stats* st) {
     gg_frontier_s* out = nullptr;
     GG_TRY(edge_map(g, F.f, f, app_threshold(g), 0, &out));
     frontier_free(out);
-    gg_frontier_s* active = nullptr;
-    if (round == 1) {
-      VPrdFirst vf{p, delta, ngh, damping, added, one_over_n, eps2};
-      GG_TRY(vertex_filter(g, All.f, vf, &active));
-    } else {
-      VPrd vf{p, delta, ngh, damping, eps2};
-      GG_TRY(vertex_filter(g, All.f, vf, &active));
-    }
-    FrontierHold A;
-    A.f = active;
+    FrontierHold A;  // the vertexFilter's output
+    GG_TRY(frontier_new(g, &A.f));
+    GG_TRY(frontier_ensure_bits(A.f, false));
+    GG_TRY(reset_stats(g));
     GG_CUDA(cudaMemsetAsync(g->ws.d_red, 0, sizeof(double), g->stream));
-    k_prd_epilogue<<<generic_grid(g, n), kGenericThreads, 0, g->stream>>>(n, delta, ngh, g->out_off(), contrib,
-                                                                          g->ws.d_red);
-    GG_CUDA(cudaGetLastError());
-    g->kernels++;
+    GG_TRY(round == 1 ? prd_vertex<true>(g, p, delta, ngh, contrib, A.f->d_bits, g->ws.d_stats)
+                      : prd_vertex<false>(g, p, delta, ngh, contrib, A.f->d_bits, g->ws.d_stats));
     double l1;
-    GG_TRY(read_red(g, &l1));
+    GG_TRY(read_stats_red(g, &l1));
+    A.f->has_dense = true;
+    A.f->dm = g->ws.h_stats[0];
+    A.f->out_edges = g->ws.h_stats[1];
     if (l1 < eps) break;
     F.reset(A.release());
   }
