@@ -131,7 +131,7 @@ __global__ void k_pr_epilogue(uint32_t n, int all, const uint32_t* fbits, float*
 // out-degree sum, L1 = sum |Delta|, nghSum reset to 0 and the next round's
 // contrib = Delta/outdeg.  It moves 32 bytes per vertex; the counts take one
 // atomic per CTA (a filter with one per warp and a separate epilogue took 18
-// us on R-MAT-20, this FIGURE).
+// us on R-MAT-20, this 8).
 template <bool FIRST>
 __global__ void __launch_bounds__(256) k_prd_vertex(uint32_t n, float* p, float* delta, float* ngh,
                                                     const uint32_t* __restrict__ off, float* contrib, uint32_t* out_bits, unsigned long long* stats,
