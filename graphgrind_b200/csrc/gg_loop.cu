@@ -768,37 +768,63 @@ static int full_occupancy(int device) {
   });
 }
 
-// Enqueues every level of the BFS from `start` as one cooperative launch
-// (k_bfs_full) on the graph's stream and returns without waiting.  `arena`
-// holds *parents and, when want_levels, *levels (n entries each) and the
-// loop's buffers.  bfs_device_full_begin_result queues the read-back of the
-// outcome, which bfs_device_full_result takes once the stream has passed it.
-int bfs_device_full(gg_graph_s* g, uint32_t start, bool want_levels, DevBuf<uint32_t>& arena, int32_t** parents,
-                    int32_t** levels, uint64_t threshold) {
-  const uint32_t n = g->n;
+// The buffers of one BFS inside its arena: *parents and, when want_levels,
+// *levels (n entries each), then the loop's own.
+struct FullBufs {
+  unsigned long long* cta;
+  int32_t *par, *lev;
+  uint32_t *q0, *q1, *eo0, *eo1, *wst0, *wst1, *bits;
+  uint32_t wstride;
+  int grid;
+  uint64_t words;  // of the whole arena
+};
+
+static int full_bufs(const gg_graph_s* g, bool want_levels, uint32_t* arena, FullBufs* out) {
   const int per_sm = full_occupancy(g->device);
   if (per_sm < 1) return fail(GG_ERR_UNSUPPORTED, "no cooperative launch of the BFS loop on this device");
   const int ctas = std::min(per_sm, g->loop_ctas_per_sm > 0 ? g->loop_ctas_per_sm : 2048 / kLoopThreads);
-  const int grid = full_grid(g->num_sms, ctas, n, g->m);
-  const uint32_t words = (n + 31) / 32;
-  const uint32_t wstride = (words + 31) & ~31u;  // 128-byte aligned bitmaps
-  const uint64_t na = ((uint64_t)n + 63) & ~63ull, wa = (g->m / kLoopThreads + 2 + 63) & ~63ull;
-  const uint64_t ca = ((uint64_t)grid * 6 + 63) & ~63ull;
-  GG_TRY(arena.alloc(g, na * (want_levels ? 6 : 5) + 2 * wa + 3ull * wstride + ca));
-  uint32_t* at = arena.p;
+  FullBufs b{};
+  b.grid = full_grid(g->num_sms, ctas, g->n, g->m);
+  b.wstride = (g->words() + 31) & ~31u;  // 128-byte aligned bitmaps
+  const uint64_t na = ((uint64_t)g->n + 63) & ~63ull, wa = (g->m / kLoopThreads + 2 + 63) & ~63ull;
   auto take = [&](uint64_t count) {
-    uint32_t* r = at;
-    at += count;
+    uint32_t* r = arena ? arena + b.words : nullptr;
+    b.words += count;
     return r;
   };
-  unsigned long long* cp = reinterpret_cast<unsigned long long*>(take(ca));
-  int32_t* par = reinterpret_cast<int32_t*>(take(na));
-  int32_t* lev = want_levels ? reinterpret_cast<int32_t*>(take(na)) : nullptr;
-  uint32_t *a0 = take(na), *a1 = take(na), *e0 = take(na), *e1 = take(na);
-  uint32_t *w0 = take(wa), *w1 = take(wa), *bp = take(3ull * wstride);
+  b.cta = reinterpret_cast<unsigned long long*>(take(((uint64_t)b.grid * 6 + 63) & ~63ull));
+  b.par = reinterpret_cast<int32_t*>(take(na));
+  if (want_levels) b.lev = reinterpret_cast<int32_t*>(take(na));
+  b.q0 = take(na);
+  b.q1 = take(na);
+  b.eo0 = take(na);
+  b.eo1 = take(na);
+  b.wst0 = take(wa);
+  b.wst1 = take(wa);
+  b.bits = take(3ull * b.wstride);
+  *out = b;
+  return GG_OK;
+}
+
+int bfs_device_full_alloc(gg_graph_s* g, bool want_levels, DevBuf<uint32_t>& arena) {
+  FullBufs b;
+  GG_TRY(full_bufs(g, want_levels, nullptr, &b));
+  return arena.alloc(g, b.words);
+}
+
+// Enqueues every level of the BFS from `start` as one cooperative launch
+// (k_bfs_full) on the graph's stream and returns without waiting; `arena` comes
+// from bfs_device_full_alloc.  bfs_device_full_begin_result queues the
+// read-back of the outcome, which bfs_device_full_result takes once the stream
+// has passed it.
+int bfs_device_full(gg_graph_s* g, uint32_t start, bool want_levels, DevBuf<uint32_t>& arena, int32_t** parents,
+                    int32_t** levels, uint64_t threshold) {
+  const uint32_t n = g->n;
+  FullBufs b;
+  GG_TRY(full_bufs(g, want_levels, arena.p, &b));
   LoopState* d_st = reinterpret_cast<LoopState*>(g->ws.d_loop);
-  k_bfs_full_init<<<generic_grid(g, n), kGenericThreads, 0, g->stream>>>(n, start, g->out_off(), par, lev, a0, e0, w0,
-                                                                         bp, 3 * wstride, d_st);
+  k_bfs_full_init<<<generic_grid(g, n), kGenericThreads, 0, g->stream>>>(n, start, g->out_off(), b.par, b.lev, b.q0,
+                                                                         b.eo0, b.wst0, b.bits, 3 * b.wstride, d_st);
   GG_CUDA(cudaGetLastError());
   const uint32_t* off = g->out_off();
   const uint32_t* idx = g->out_idx();
@@ -806,24 +832,27 @@ int bfs_device_full(gg_graph_s* g, uint32_t start, bool want_levels, DevBuf<uint
   // the bottom-up levels walk the in-lists hub sources first (same edges,
   // other order: a vertex then meets a frontier in-neighbour sooner)
   // (graphs the copy cannot be built for, past 2^31 edges or without the
-  // memory, walk the CSC's own in-lists)
-  if (g->early_kernel == 3 && !g->d_bu_idx && build_bu_index(g) != GG_OK) cudaGetLastError();
+  // memory, walk the CSC's own in-lists).  The copy costs a segmented sort of
+  // all edges and its temporaries (R-MAT-22: 17 ms against a traversal of
+  // 0.2 ms), so the first BFS of a graph walks the CSC's in-lists too.
+  if (g->early_kernel == 3 && !g->d_bu_idx && g->bfs_ran && build_bu_index(g) != GG_OK) cudaGetLastError();
+  g->bfs_ran = true;
   const uint32_t* iidx = g->early_kernel == 3 && g->d_bu_idx ? g->d_bu_idx : g->in_idx();
-  uint32_t ws = wstride, nn = n;
+  uint32_t nn = n;
   int32_t round0 = 1;
   unsigned long long thr = threshold;
   int32_t cap = n < (uint32_t)INT32_MAX ? (int32_t)n + 1 : INT32_MAX;
   unsigned budget = g->loop_wait_budget;
   int vec = g->early_kernel >= 2 ? 1 : 0, mark = 0;
   unsigned long long handover = 0;
-  void* args[] = {(void*)&off, (void*)&idx, (void*)&ioff, (void*)&iidx, (void*)&par,  (void*)&lev,
-                  (void*)&a0,  (void*)&a1,  (void*)&e0,   (void*)&e1,   (void*)&w0,   (void*)&w1,
-                  (void*)&bp,  (void*)&ws,  (void*)&cp,   (void*)&nn,   (void*)&d_st, (void*)&round0,
-                  (void*)&thr, (void*)&cap, (void*)&budget, (void*)&vec, (void*)&mark, (void*)&handover};
-  GG_CUDA(cudaLaunchCooperativeKernel((const void*)k_bfs_full, grid, kLoopThreads, args, 0, g->stream));
+  void* args[] = {(void*)&off,    (void*)&idx,    (void*)&ioff,   (void*)&iidx,   (void*)&b.par,  (void*)&b.lev,
+                  (void*)&b.q0,   (void*)&b.q1,   (void*)&b.eo0,  (void*)&b.eo1,  (void*)&b.wst0, (void*)&b.wst1,
+                  (void*)&b.bits, (void*)&b.wstride, (void*)&b.cta, (void*)&nn,   (void*)&d_st,   (void*)&round0,
+                  (void*)&thr,    (void*)&cap,    (void*)&budget, (void*)&vec,    (void*)&mark,   (void*)&handover};
+  GG_CUDA(cudaLaunchCooperativeKernel((const void*)k_bfs_full, b.grid, kLoopThreads, args, 0, g->stream));
   g->kernels += 2;
-  *parents = par;
-  *levels = lev;
+  *parents = b.par;
+  *levels = b.lev;
   return GG_OK;
 }
 

@@ -420,7 +420,7 @@ int gg_graph_set_dense_policy(gg_graph_t g, int32_t policy);
  *                         GG_TUNE_DEVICE_LOOP 2 walk a copy of the in-lists
  *                         with each list's sources by descending out-degree
  *                         (a vertex meets a frontier in-neighbour sooner:
- *                         0.438 against 0.452 ms); the first such BFS builds
+ *                         0.438 against 0.452 ms); the second such BFS builds
  *                         the copy (one segmented sort), which stays with the
  *                         graph: 4 bytes per edge (a graph past 2^31 edges,
  *                         or one the copy does not fit beside, walks the
