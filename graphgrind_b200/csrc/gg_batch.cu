@@ -17,101 +17,105 @@
 
 namespace gg {
 
-// Sum pull: S[v, c] = sum over in-edges u->v of XS[u, c], for c in one
-// 32-column slab per lane pair.  One warp per 256-edge block of the CSC; the
-// head-bit row structure tells every edge's row.  Rows that end inside the
-// block are stored; rows that cross a block boundary are added atomically
-// (those rows were zeroed before the launch).
-template <int KW>  // KW = columns per lane (1 -> 32 columns, 2 -> 64 columns)
-__global__ void __launch_bounds__(256) k_ppr_pull(const uint32_t* idx, const uint32_t* head, const uint32_t* blk,
-                                                   const uint32_t* rows, uint64_t nblocks, uint64_t m,
-                                                   const float* xs, float* S, uint32_t k) {
-  __shared__ uint32_t s_idx[8][kSegBlock];
-  __shared__ uint8_t s_head[8][kSegBlock];
+// Sum pull: S[v, c] = sum over in-edges u->v of XS[u, c].  One warp per
+// 256-edge block of the CSC, split into SUBS = 128 / K groups of lanes: each
+// group takes a contiguous share of the block's edges (a segment), a lane four
+// of the K columns, so that one 16-byte load instruction of the warp gathers
+// SUBS whole rows.  What bounds the pull is how many gathered bytes are in
+// flight (4K an edge, from L2): 8 rows per group before any is used (64
+// columns, R-MAT-18: 123 us with a warp per row and 8 bytes per lane, 74
+// us now).  The head-bit row structure tells every edge's row.  Rows that end
+// inside their segment are stored; rows that cross a segment boundary are added
+// atomically (those rows were zeroed before the launch).
+template <int K>
+struct PprShape {
+  static constexpr int kLanes = K / 4;            // lanes per edge
+  static constexpr int kSubs = 32 / kLanes;       // edges per load instruction
+  static constexpr int kSeg = kSegBlock / kSubs;  // edges of a segment (64 or 128)
+};
+
+template <int K>
+__global__ void __launch_bounds__(256) k_ppr_pull(const uint32_t* __restrict__ idx, const uint32_t* __restrict__ head,
+                                                  const uint32_t* __restrict__ blk, const uint32_t* __restrict__ rows,
+                                                  uint64_t nblocks, uint64_t m, const float* __restrict__ xs,
+                                                  float* S) {
+  using Sh = PprShape<K>;
+  __shared__ __align__(16) uint32_t s_idx[8][kSegBlock];
+  __shared__ uint32_t s_hw[8][9];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int sub = lane / Sh::kLanes, col = (lane % Sh::kLanes) * 4;
   const uint64_t warps = (uint64_t)gridDim.x * (blockDim.x >> 5);
   for (uint64_t b = (uint64_t)blockIdx.x * (blockDim.x >> 5) + warp; b < nblocks; b += warps) {
     const uint64_t e0 = b * kSegBlock;
-    // stage this block's sources and row-head flags (lane l: edges 8l .. 8l+7)
-    const uint4 ia = __ldg(reinterpret_cast<const uint4*>(idx + e0) + 2 * lane);
-    const uint4 ib = __ldg(reinterpret_cast<const uint4*>(idx + e0) + 2 * lane + 1);
-    const uint32_t hw = __ldg(head + b * 8 + (lane >> 2));
-    const uint32_t bits = (hw >> ((lane & 3) * 8)) & 0xffu;
-    reinterpret_cast<uint4*>(s_idx[warp])[2 * lane] = ia;
-    reinterpret_cast<uint4*>(s_idx[warp])[2 * lane + 1] = ib;
-#pragma unroll
-    for (int q = 0; q < 8; ++q) s_head[warp][lane * 8 + q] = (bits >> q) & 1u;
+    // this block's sources and head bits (with the next block's first word)
+    reinterpret_cast<uint4*>(s_idx[warp])[2 * lane] = __ldg(reinterpret_cast<const uint4*>(idx + e0) + 2 * lane);
+    reinterpret_cast<uint4*>(s_idx[warp])[2 * lane + 1] = __ldg(reinterpret_cast<const uint4*>(idx + e0) + 2 * lane + 1);
+    const bool more = e0 + kSegBlock < m;
+    if (lane < 8 || (lane == 8 && more)) s_hw[warp][lane] = __ldg(head + b * 8 + lane);
     __syncwarp();
     const uint32_t blk_end = m - e0 < (uint64_t)kSegBlock ? (uint32_t)(m - e0) : (uint32_t)kSegBlock;
-    // the row continuing from the previous block has ordinal blk[b] - 1
-    uint32_t cur_ord = __ldg(blk + b) - 1u;
-    bool started_here = false;
-    int have = 0;
-    float acc[KW];
-#pragma unroll
-    for (int c = 0; c < KW; ++c) acc[c] = 0.f;
+    const uint32_t beg = min(blk_end, (uint32_t)(sub * Sh::kSeg)), end = min(blk_end, beg + (uint32_t)Sh::kSeg);
+    // the row that continues into the segment: heads before it, less one
+    uint32_t ord = __ldg(blk + b) - 1u;
+    for (int w = 0; w < sub * Sh::kSeg / 32; ++w) ord += __popc(s_hw[warp][w]);
+    bool started = false;
+    bool have = false;
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
     auto flush = [&](bool complete) {
-      float* dst = S + (uint64_t)__ldg(rows + cur_ord) * k + lane * KW;
-      if (complete) {
-#pragma unroll
-        for (int c = 0; c < KW; ++c) dst[c] = acc[c];
-      } else {
-#pragma unroll
-        for (int c = 0; c < KW; ++c) atomicAdd(dst + c, acc[c]);
-      }
+      float4* dst = reinterpret_cast<float4*>(S + (uint64_t)__ldg(rows + ord) * K + col);
+      if (complete)
+        *dst = acc;
+      else
+        atomicAdd(dst, acc);
     };
-    for (uint32_t g0 = 0; g0 < blk_end; g0 += 8) {
+    for (uint32_t g0 = beg; g0 < end; g0 += 8) {
       // issue the group's row gathers before consuming them
-      float v[8][KW];
+      float4 v[8];
+#pragma unroll
+      for (int q = 0; q < 8; ++q)
+        if (g0 + q < end)
+          v[q] = __ldg(reinterpret_cast<const float4*>(xs + (uint64_t)s_idx[warp][g0 + q] * K + col));
+      const uint32_t bits = (s_hw[warp][g0 >> 5] >> (g0 & 31)) & 0xffu;
 #pragma unroll
       for (int q = 0; q < 8; ++q) {
-        const uint32_t e = g0 + q;
-        if (e < blk_end) {
-          const float* xr = xs + (uint64_t)s_idx[warp][e] * k + lane * KW;
-          if (KW == 2) {
-            const float2 t = __ldg(reinterpret_cast<const float2*>(xr));
-            v[q][0] = t.x;
-            v[q][KW - 1] = t.y;
-          } else {
-            v[q][0] = __ldg(xr);
-          }
+        if (g0 + q >= end) break;
+        if ((bits >> q) & 1u) {  // a new row starts: the current one is done
+          if (have) flush(started);
+          ++ord;
+          started = true;
+          acc = make_float4(0.f, 0.f, 0.f, 0.f);
         }
-      }
-#pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        const uint32_t e = g0 + q;
-        if (e >= blk_end) break;
-        if (s_head[warp][e]) {  // a new row starts: the current one is done
-          if (have > 0) flush(started_here);
-          ++cur_ord;
-          started_here = true;
-          have = 0;
-#pragma unroll
-          for (int c = 0; c < KW; ++c) acc[c] = 0.f;
-        }
-#pragma unroll
-        for (int c = 0; c < KW; ++c) acc[c] += v[q][c];
-        ++have;
+        acc.x += v[q].x;
+        acc.y += v[q].y;
+        acc.z += v[q].z;
+        acc.w += v[q].w;
+        have = true;
       }
     }
-    if (have > 0) {  // the last row is complete only if the next block starts a new row
-      const uint64_t nxt = e0 + blk_end;
-      const bool ends_here = nxt >= m || ((__ldg(head + (nxt >> 5)) >> (nxt & 31)) & 1u);
-      flush(started_here && ends_here);
+    if (have) {  // the last row is complete only if a row starts right after the segment
+      const bool ends_here = e0 + end >= m || ((s_hw[warp][end >> 5] >> (end & 31)) & 1u);
+      flush(started && ends_here);
     }
     __syncwarp();
   }
 }
 
-// The rows that cross a 256-edge block boundary (they receive partial sums):
-// row_list[0 .. *count).  The row that continues into block b is listed by the
-// first block it continues into.
-__global__ void k_boundary_rows(const uint32_t* head, const uint32_t* blk, const uint32_t* rows, uint64_t nblocks,
-                                uint32_t* row_list, uint32_t* count) {
-  for (uint64_t b = 1 + (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; b < nblocks;
-       b += (uint64_t)gridDim.x * blockDim.x) {
-    const uint32_t h = blk[b];
-    if (!(head[b * 8] & 1u) && h != blk[b - 1]) row_list[atomicAdd(count, 1u)] = rows[h - 1];
+// The rows that cross a segment boundary (they receive partial sums):
+// row_list[0 .. *count).  The row that continues into a segment is listed by
+// the first segment it continues into.  segs: segments of seg edges in the
+// stream.
+__global__ void k_boundary_rows(const uint32_t* head, const uint32_t* blk, const uint32_t* rows, uint64_t segs,
+                                uint32_t seg, uint32_t* row_list, uint32_t* count) {
+  for (uint64_t t = 1 + (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; t < segs;
+       t += (uint64_t)gridDim.x * blockDim.x) {
+    const uint64_t w = t * (seg / 32);  // the segment's first head word
+    if (head[w] & 1u) continue;
+    bool before = false;  // a row starts in the segment before this one
+    for (uint32_t i = 1; i <= seg / 32; ++i) before |= head[w - i] != 0;
+    if (!before) continue;
+    uint32_t ord = blk[w / 8] - 1u;
+    for (uint64_t i = w / 8 * 8; i < w; ++i) ord += __popc(head[i]);
+    row_list[atomicAdd(count, 1u)] = rows[ord];
   }
 }
 
@@ -217,26 +221,26 @@ static int ppr_columns(gg_graph_s* g, uint32_t k, int32_t iters, float damping, 
   const int ksh = k == 64 ? 6 : 5, vgrid = generic_grid(g, total4);
   const int pgrid = (int)std::max<uint64_t>(1, std::min<uint64_t>((nblocks + 7) / 8, (uint64_t)g->num_sms * 16));
   DevBuf<uint32_t> brows;  // the count, then the rows
-  GG_TRY(brows.alloc(g, nblocks + 4));
+  const uint32_t seg = k == 64 ? PprShape<64>::kSeg : PprShape<32>::kSeg;
+  const uint64_t segs = (g->m + seg - 1) / seg;
+  GG_TRY(brows.alloc(g, segs + 4));
   GG_CUDA(cudaMemsetAsync(brows.p, 0, 4, g->stream));
   GG_CUDA(cudaMemsetAsync(S, 0, 4ull * g->n * k, g->stream));  // rows without in-edges stay 0
-  k_boundary_rows<<<generic_grid(g, std::max<uint64_t>(nblocks, 1)), kGenericThreads, 0, g->stream>>>(
-      si.d_head, si.d_blk, si.d_rows, nblocks, brows.p + 4, brows.p);
+  k_boundary_rows<<<generic_grid(g, std::max<uint64_t>(segs, 1)), kGenericThreads, 0, g->stream>>>(
+      si.d_head, si.d_blk, si.d_rows, segs, seg, brows.p + 4, brows.p);
   k_ppr_rows<<<vgrid, kGenericThreads, 0, g->stream>>>(total4, ksh, g->in_off(), g->out_off(), S, T, tbits, damping, XS, 1,
                                                        iters == 0);
   g->kernels += 2;
   for (int32_t it = 0; it < iters; ++it) {
     if (nblocks) {
       if (it > 0) {
-        k_zero_rows<<<generic_grid(g, nblocks * k), kGenericThreads, 0, g->stream>>>(brows.p + 4, brows.p, S, k);
+        k_zero_rows<<<generic_grid(g, segs * k), kGenericThreads, 0, g->stream>>>(brows.p + 4, brows.p, S, k);
         g->kernels++;
       }
       if (k == 64)
-        k_ppr_pull<2><<<pgrid, 256, 0, g->stream>>>(g->in_idx(), si.d_head, si.d_blk, si.d_rows, nblocks, g->m, XS, S,
-                                                    k);
+        k_ppr_pull<64><<<pgrid, 256, 0, g->stream>>>(g->in_idx(), si.d_head, si.d_blk, si.d_rows, nblocks, g->m, XS, S);
       else
-        k_ppr_pull<1><<<pgrid, 256, 0, g->stream>>>(g->in_idx(), si.d_head, si.d_blk, si.d_rows, nblocks, g->m, XS, S,
-                                                    k);
+        k_ppr_pull<32><<<pgrid, 256, 0, g->stream>>>(g->in_idx(), si.d_head, si.d_blk, si.d_rows, nblocks, g->m, XS, S);
       g->kernels++;
     }
     k_ppr_rows<<<vgrid, kGenericThreads, 0, g->stream>>>(total4, ksh, g->in_off(), g->out_off(), S, T, tbits, damping, XS, 0,
