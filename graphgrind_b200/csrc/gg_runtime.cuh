@@ -645,7 +645,11 @@ int edge_map(gg_graph_s* g, gg_frontier_s* in, const F& f, int64_t threshold, ui
     } else if (!in->bit && !in->has_dense) {
       rc = frontier_to_dense(in);
     }
-    if (!rc) rc = frontier_ensure_bits(o, true);
+    // an output nobody reads from the kernels that have a form without one
+    // (pull_launch: 1, 6 and 7, whose direct loads cannot set the error word
+    // either): no bitmap to clear and no statistics to read
+    const bool bare = no_out && !g->coo_by_source && (g->coo_kernel == 1 || g->coo_kernel >= 6);
+    if (!rc && !bare) rc = frontier_ensure_bits(o, true);
     if (!rc) rc = reset_stats(g);
     if (!rc) {
       prof_begin();
@@ -658,14 +662,16 @@ int edge_map(gg_graph_s* g, gg_frontier_s* in, const F& f, int64_t threshold, ui
                 : pull_launch<F, false>(g, in, o, f, coo_pull, no_out);
       if (g->profiling) cudaEventRecord(g->prof_ev[1], g->stream);
     }
-    // an output nobody reads from a pull without waits (the direct-load COO
-    // kernels; only the bulk-copy rings, 0/2/3, can set the error word), for
-    // an application that synchronises later itself (kEmNoWait): no
-    // statistics to read, and the stream goes on without a host round trip
+    // for an application that synchronises later itself (kEmNoWait), the
+    // stream goes on without a host round trip (only the bulk-copy rings,
+    // 0/2/3, can set the error word)
     const bool skip_stats = no_out && (flags & kEmNoWait) && g->coo_kernel != 0 && g->coo_kernel != 2 &&
                             g->coo_kernel != 3;
     if (!rc && skip_stats && g->profiling) {
       if (cudaEventSynchronize(g->prof_ev[1]) != cudaSuccess) rc = fail(GG_ERR_CUDA, "edgeMap: profiling event");
+    } else if (!rc && bare && !skip_stats) {
+      const cudaError_t e = cudaStreamSynchronize(g->stream);
+      if (e != cudaSuccess) rc = fail(GG_ERR_CUDA, "edgeMap: %s", cudaGetErrorString(e));
     } else if (!rc && !skip_stats) {
       rc = read_stats(g);
     }
