@@ -349,7 +349,8 @@ int pull_launch(gg_graph_s* g, gg_frontier_s* in, gg_frontier_s* out, const F& f
   if (coo && g->coo_kernel > 0) {  // per-warp COO pull: 0, 2 or 3 staging stages
     static DeviceOnce opted[2][4];
     static DeviceOnce opted_pf[2];
-    static DeviceOnce opted_no[3][2];
+    static DeviceOnce opted_no[4][2];
+    const bool split = g->d_coo_slab != nullptr;  // some tile is cut into several work items
     static DeviceOnce opted_mg[2];
     constexpr int kFlags = coo_w_flag_bytes<F, false>(), kFlagsNoOut = coo_w_flag_bytes<F, true>();
     auto launch_w = [&](auto kern, int stages, DeviceOnce& once, int flags) -> int {
@@ -379,17 +380,27 @@ int pull_launch(gg_graph_s* g, gg_frontier_s* in, gg_frontier_s* out, const F& f
         return all ? launch_w(k_pull_coo_w<F, kHW, true, 0, false, false, true, true>, 0, opted_no[1][1], kFlagsNoOut)
                    : launch_w(k_pull_coo_w<F, kHW, false, 0, false, false, true, true>, 0, opted_no[1][0],
                               kFlagsNoOut);
-      if (no_out && g->coo_kernel == 7)
+      if (no_out && g->coo_kernel == 7 && split)
         return all ? launch_w(k_pull_coo_w<F, kHW, true, 0, false, false, true, true, 3>, 0, opted_no[2][1],
                               kFlagsNoOut)
                    : launch_w(k_pull_coo_w<F, kHW, false, 0, false, false, true, true, 3>, 0, opted_no[2][0],
                               kFlagsNoOut);
+      if (no_out && g->coo_kernel == 7)
+        return all ? launch_w(k_pull_coo_w<F, kHW, true, 0, false, false, true, true, 3, false>, 0, opted_no[3][1],
+                              kFlagsNoOut)
+                   : launch_w(k_pull_coo_w<F, kHW, false, 0, false, false, true, true, 3, false>, 0, opted_no[3][0],
+                              kFlagsNoOut);
     }
-    static DeviceOnce opted_h[2];
+    static DeviceOnce opted_h[2][2];
     switch (g->coo_kernel) {
       case 7:
-        return all ? launch_w(k_pull_coo_w<F, kHW, true, 0, false, false, false, true, 7>, 0, opted_h[1], kFlags)
-                   : launch_w(k_pull_coo_w<F, kHW, false, 0, false, false, false, true, 7>, 0, opted_h[0], kFlags);
+        if (!split)
+          return all ? launch_w(k_pull_coo_w<F, kHW, true, 0, false, false, false, true, 7, false>, 0, opted_h[1][1],
+                                kFlags)
+                     : launch_w(k_pull_coo_w<F, kHW, false, 0, false, false, false, true, 7, false>, 0, opted_h[1][0],
+                                kFlags);
+        return all ? launch_w(k_pull_coo_w<F, kHW, true, 0, false, false, false, true, 7>, 0, opted_h[0][1], kFlags)
+                   : launch_w(k_pull_coo_w<F, kHW, false, 0, false, false, false, true, 7>, 0, opted_h[0][0], kFlags);
       case 6:
         return all ? launch_w(k_pull_coo_w<F, kHW, true, 0, false, false, false, true>, 0, opted_mg[1], kFlags)
                    : launch_w(k_pull_coo_w<F, kHW, false, 0, false, false, false, true>, 0, opted_mg[0], kFlags);
