@@ -10,9 +10,9 @@
 // first) and finish each inside the CTA without grid barriers: its
 // level-synchronous top-down traversal of app/BFS.C:77-101 balances a
 // frontier's edges over the CTA's threads by a block prefix sum over the
-// frontier's degrees.  Batches past 2^31 vertices or 2^32 edges run in that
-// kernel alone.  The launch sequence is captured once as a CUDA graph and
-// replayed.
+// frontier's degrees.  Batches past 2^31 vertices or 2^32 edges, and those whose
+// in-edges do not fit beside them, run in that kernel alone.  The launch
+// sequence is captured once as a CUDA graph and replayed.
 #include <cub/cub.cuh>
 
 #include <algorithm>
@@ -40,7 +40,8 @@ struct gg_graph_batch_s {
   uint64_t total_n = 0, total_m = 0;
   uint32_t max_n = 0;
   std::vector<uint64_t> firsts;
-  bool whole = false;  // one union graph (else local ids, one CTA per graph)
+  bool whole = false;  // union ids in the arenas (else every graph counts from 0)
+  bool loop = false;   // the union's in-edges and loop buffers exist: the loop runs first (else one CTA per graph alone)
   int num_sms = 0;
   gg::UnionBfs uni;
   uint32_t *d_ioff = nullptr, *d_iidx = nullptr;
@@ -129,7 +130,7 @@ __global__ void __launch_bounds__(kBatchThreads) k_batch_bfs(const BatchDesc* __
     } else {
       for (uint32_t v = tid; v < d.n; v += kBatchThreads) lev[v] = -1;
       __syncthreads();
-      const uint32_t s = src[gi];
+      const uint32_t s = src[gi] - d.vfirst;
       if (tid == 0) {
         lev[s] = 0;
         qa[0] = s;
@@ -327,15 +328,24 @@ static int batch_build(int32_t count, const gg_host_graph* graphs, gg_graph_batc
     GG_CUDA(cudaMemcpy(d_first, edge_first.data(), 8 * ((uint64_t)count + 1), cudaMemcpyHostToDevice));
     k_batch_globalise<<<std::min(count, b->num_sms * 8), 256, 0, b->stream>>>(b->d_desc, d_first, count, b->d_idx);
     GG_CUDA(cudaGetLastError());
-    GG_TRY(batch_in_edges(b, (uint32_t)b->total_n));
     b->uni.off = b->d_off;
     b->uni.idx = b->d_idx;
-    b->uni.ioff = b->d_ioff;
-    b->uni.iidx = b->d_iidx;
     b->uni.levels = b->d_levels;
     b->uni.n = (uint32_t)b->total_n;
     b->uni.m = b->total_m;
-    GG_TRY(union_bfs_prepare(b->uni, b->device, b->num_sms));
+    // a batch whose in-edges or loop buffers do not fit beside it keeps one
+    // CTA per graph
+    b->loop = batch_in_edges(b, (uint32_t)b->total_n) == GG_OK;
+    b->uni.ioff = b->d_ioff;
+    b->uni.iidx = b->d_iidx;
+    b->loop = b->loop && union_bfs_prepare(b->uni, b->device, b->num_sms) == GG_OK;
+    if (!b->loop) {
+      cudaGetLastError();
+      union_bfs_free(b->uni);
+      cudaFree(b->d_ioff);
+      cudaFree(b->d_iidx);
+      b->d_ioff = b->d_iidx = nullptr;
+    }
   }
   std::vector<uint32_t> order(count);
   std::iota(order.begin(), order.end(), 0u);
@@ -352,12 +362,12 @@ static int batch_build(int32_t count, const gg_host_graph* graphs, gg_graph_batc
   GG_CUDA(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
   cudaMemcpyAsync(b->d_src, b->h_src, 4 * count, cudaMemcpyHostToDevice, b->stream);
   cudaMemsetAsync(b->d_ctr, 0, 16, b->stream);
-  if (b->whole) GG_TRY(union_bfs_enqueue(b->uni, b->stream, b->num_sms, b->d_src, (uint32_t)count));
+  if (b->loop) GG_TRY(union_bfs_enqueue(b->uni, b->stream, b->num_sms, b->d_src, (uint32_t)count));
   k_batch_bfs<<<b->grid, kBatchThreads, 0, b->stream>>>(b->d_desc, b->d_order, count, b->d_off, b->d_idx,
                                                           b->d_levels, b->d_src, b->d_ctr, b->d_scratch, b->max_n,
-                                                          b->whole ? b->uni.st : nullptr);
+                                                          b->loop ? b->uni.st : nullptr);
   cudaMemcpyAsync(b->h_ctr, b->d_ctr, 16, cudaMemcpyDeviceToHost, b->stream);
-  if (b->whole)
+  if (b->loop)
     cudaMemcpyAsync(b->h_ctr + 2, b->uni.st, sizeof(LoopState), cudaMemcpyDeviceToHost, b->stream);
   GG_CUDA(cudaStreamEndCapture(b->stream, &b->graph));
   GG_CUDA(cudaGraphInstantiate(&b->exec, b->graph, 0));
@@ -441,15 +451,15 @@ int gg_batch_bfs(gg_graph_batch_t b, const uint32_t* sources, int32_t* levels, g
   GG_CUDA(cudaStreamSynchronize(b->stream));
   GG_CUDA(cudaGetLastError());
   const LoopState* loop = reinterpret_cast<const LoopState*>(b->h_ctr + 2);
-  if (b->whole && loop->exit_reason < 0) return fail(GG_ERR_TIMEOUT, "gg_batch_bfs: a grid barrier wait ran out");
-  if (b->whole && loop->exit_reason != 1 && loop->exit_reason != 4)
+  if (b->loop && loop->exit_reason < 0) return fail(GG_ERR_TIMEOUT, "gg_batch_bfs: a grid barrier wait ran out");
+  if (b->loop && loop->exit_reason != 1 && loop->exit_reason != 4)
     return fail(GG_ERR_CUDA, "gg_batch_bfs: stopped without an empty frontier (reason %d)", loop->exit_reason);
   if (levels && down != levels) std::copy(b->h_levels, b->h_levels + b->total_n, levels);
   if (st) {
     st->ms = ms;
     st->rounds = 1;
-    st->edges_traversed = b->h_ctr[1] + (b->whole ? loop->trav : 0);
-    st->kernels = b->whole ? 4 : 1;
+    st->edges_traversed = b->h_ctr[1] + (b->loop ? loop->trav : 0);
+    st->kernels = b->loop ? 4 : 1;
   }
   return GG_OK;
 }
