@@ -283,7 +283,7 @@ static int run_bfs(gg_graph_s* g, uint32_t start, int32_t* parents, int32_t* lev
   // writes levels only when they are asked for
   const bool full = g->device_loop == 2 && !g->transposed && g->dense_policy != 2;
   // before anything is queued: mapping new memory waits for the device
-  if (full) GG_TRY(bfs_device_full_alloc(g, levels != nullptr, arena));
+  if (full) GG_TRY(bfs_device_full_prepare(g, levels != nullptr, arena));
   EventTimer tm(g->stream);
   FrontierHold F;
   int32_t round = 0;

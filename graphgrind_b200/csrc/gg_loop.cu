@@ -806,15 +806,24 @@ static int full_bufs(const gg_graph_s* g, bool want_levels, uint32_t* arena, Ful
   return GG_OK;
 }
 
-int bfs_device_full_alloc(gg_graph_s* g, bool want_levels, DevBuf<uint32_t>& arena) {
+int bfs_device_full_prepare(gg_graph_s* g, bool want_levels, DevBuf<uint32_t>& arena) {
   FullBufs b;
   GG_TRY(full_bufs(g, want_levels, nullptr, &b));
-  return arena.alloc(g, b.words);
+  GG_TRY(arena.alloc(g, b.words));
+  // the bottom-up levels walk the in-lists hub sources first (same edges,
+  // other order: a vertex then meets a frontier in-neighbour sooner)
+  // (graphs the copy cannot be built for, past 2^31 edges or without the
+  // memory, walk the CSC's own in-lists).  The copy costs a segmented sort of
+  // all edges and its temporaries (R-MAT-22: 17 ms against a traversal of
+  // 0.2 ms), so the first BFS of a graph walks the CSC's in-lists too.
+  if (g->early_kernel == 3 && !g->d_bu_idx && g->bfs_ran && build_bu_index(g) != GG_OK) cudaGetLastError();
+  g->bfs_ran = true;
+  return GG_OK;
 }
 
 // Enqueues every level of the BFS from `start` as one cooperative launch
 // (k_bfs_full) on the graph's stream and returns without waiting; `arena` comes
-// from bfs_device_full_alloc.  bfs_device_full_begin_result queues the
+// from bfs_device_full_prepare.  bfs_device_full_begin_result queues the
 // read-back of the outcome, which bfs_device_full_result takes once the stream
 // has passed it.
 int bfs_device_full(gg_graph_s* g, uint32_t start, bool want_levels, DevBuf<uint32_t>& arena, int32_t** parents,
@@ -829,14 +838,6 @@ int bfs_device_full(gg_graph_s* g, uint32_t start, bool want_levels, DevBuf<uint
   const uint32_t* off = g->out_off();
   const uint32_t* idx = g->out_idx();
   const uint32_t* ioff = g->in_off();
-  // the bottom-up levels walk the in-lists hub sources first (same edges,
-  // other order: a vertex then meets a frontier in-neighbour sooner)
-  // (graphs the copy cannot be built for, past 2^31 edges or without the
-  // memory, walk the CSC's own in-lists).  The copy costs a segmented sort of
-  // all edges and its temporaries (R-MAT-22: 17 ms against a traversal of
-  // 0.2 ms), so the first BFS of a graph walks the CSC's in-lists too.
-  if (g->early_kernel == 3 && !g->d_bu_idx && g->bfs_ran && build_bu_index(g) != GG_OK) cudaGetLastError();
-  g->bfs_ran = true;
   const uint32_t* iidx = g->early_kernel == 3 && g->d_bu_idx ? g->d_bu_idx : g->in_idx();
   uint32_t nn = n;
   int32_t round0 = 1;

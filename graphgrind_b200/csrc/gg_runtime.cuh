@@ -262,7 +262,7 @@ int frontier_to_sparse(gg_frontier_s* f);
 void frontier_free(gg_frontier_s* f);
 int bfs_device_levels(gg_graph_s* g, gg_frontier_s** F, int32_t* parents, int32_t* levels, int32_t round0,
                       uint64_t threshold, int32_t* rounds, uint64_t* trav);
-int bfs_device_full_alloc(gg_graph_s* g, bool want_levels, DevBuf<uint32_t>& arena);
+int bfs_device_full_prepare(gg_graph_s* g, bool want_levels, DevBuf<uint32_t>& arena);
 int bfs_device_full(gg_graph_s* g, uint32_t start, bool want_levels, DevBuf<uint32_t>& arena, int32_t** parents,
                     int32_t** levels, uint64_t threshold);
 int bfs_device_full_begin_result(gg_graph_s* g);
