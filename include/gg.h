@@ -595,7 +595,7 @@ int gg_msbc(gg_graph_t g, int32_t k, const uint32_t* sources, float* dependencie
 /* ======================================================== many graphs */
 /* No single counterpart in the reference (one graph per process there).  A
  * batch of independent graphs of uneven size held in one device arena, for
- * running one traversal over all of them in a single persistent launch. */
+ * running one traversal over all of them in a single call. */
 typedef struct gg_graph_batch_s* gg_graph_batch_t;
 /* Uploads `count` host graphs (out-edge CSR each; weights ignored). */
 int gg_batch_create(int32_t count, const gg_host_graph* graphs, gg_graph_batch_t* out);
