@@ -272,6 +272,15 @@ static int batch_in_edges(gg_graph_batch_s* b, uint32_t n) {
   return GG_OK;
 }
 
+// Host data to the device in the order of the batch's stream.  That stream does
+// not wait for the default stream, in which a plain copy of pageable memory may
+// still be under way when the call returns.
+template <class T>
+static int upload(gg_graph_batch_s* b, T* dst, const T* src, uint64_t count) {
+  GG_CUDA(cudaMemcpyAsync(dst, src, sizeof(T) * count, cudaMemcpyHostToDevice, b->stream));
+  return GG_OK;
+}
+
 static int batch_build(int32_t count, const gg_host_graph* graphs, gg_graph_batch_s* b) {
   b->count = count;
   std::vector<BatchDesc> desc(count);
@@ -303,7 +312,7 @@ static int batch_build(int32_t count, const gg_host_graph* graphs, gg_graph_batc
   GG_CUDA(cudaMalloc(&b->d_order, 4 * count));
   GG_CUDA(cudaMalloc(&b->d_src, 4 * count));
   GG_CUDA(cudaMalloc(&b->d_ctr, 16));
-  GG_CUDA(cudaMemcpy(b->d_desc, desc.data(), sizeof(BatchDesc) * count, cudaMemcpyHostToDevice));
+  GG_TRY(upload(b, b->d_desc, desc.data(), count));
   {
     std::vector<uint32_t> off(offs);
 #pragma omp parallel for schedule(dynamic, 8)
@@ -313,11 +322,11 @@ static int batch_build(int32_t count, const gg_host_graph* graphs, gg_graph_batc
       for (uint64_t v = 0; v < (uint64_t)h.n + (b->whole ? 0 : 1); ++v) off[desc[i].off_base + v] = h.offsets[v] + base;
     }
     if (b->whole) off[b->total_n] = (uint32_t)b->total_m;
-    GG_CUDA(cudaMemcpy(b->d_off, off.data(), 4 * offs, cudaMemcpyHostToDevice));
+    GG_TRY(upload(b, b->d_off, off.data(), offs));
+    GG_CUDA(cudaStreamSynchronize(b->stream));  // off leaves scope
   }
   for (int32_t i = 0; i < count; ++i)
-    if (graphs[i].m)
-      GG_CUDA(cudaMemcpy(b->d_idx + edge_first[i], graphs[i].indices, 4 * graphs[i].m, cudaMemcpyHostToDevice));
+    if (graphs[i].m) GG_TRY(upload<uint32_t>(b, b->d_idx + edge_first[i], graphs[i].indices, graphs[i].m));
   if (b->whole) {
     uint64_t* d_first = nullptr;
     GG_CUDA(cudaMalloc(&d_first, 8 * ((uint64_t)count + 1)));
@@ -325,7 +334,7 @@ static int batch_build(int32_t count, const gg_host_graph* graphs, gg_graph_batc
       void* p;
       ~Hold() { cudaFree(p); }
     } hold{d_first};
-    GG_CUDA(cudaMemcpy(d_first, edge_first.data(), 8 * ((uint64_t)count + 1), cudaMemcpyHostToDevice));
+    GG_TRY(upload(b, d_first, edge_first.data(), (uint64_t)count + 1));
     k_batch_globalise<<<std::min(count, b->num_sms * 8), 256, 0, b->stream>>>(b->d_desc, d_first, count, b->d_idx);
     GG_CUDA(cudaGetLastError());
     b->uni.off = b->d_off;
@@ -350,7 +359,8 @@ static int batch_build(int32_t count, const gg_host_graph* graphs, gg_graph_batc
   std::vector<uint32_t> order(count);
   std::iota(order.begin(), order.end(), 0u);
   std::stable_sort(order.begin(), order.end(), [&](uint32_t x, uint32_t y) { return graphs[x].m > graphs[y].m; });
-  GG_CUDA(cudaMemcpy(b->d_order, order.data(), 4 * count, cudaMemcpyHostToDevice));
+  GG_TRY(upload(b, b->d_order, order.data(), count));
+  GG_CUDA(cudaStreamSynchronize(b->stream));  // the host arrays are the caller's and this function's
   int per_sm = 0;
   GG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batch_bfs, kBatchThreads, 0));
   b->grid = std::max(1, std::min(count, b->num_sms * std::max(per_sm, 1)));
