@@ -38,6 +38,7 @@ struct gg_graph_batch_s {
   cudaStream_t stream = nullptr;
   int32_t count = 0;
   uint64_t total_n = 0, total_m = 0;
+  uint64_t edges = 0;  // edges in the arena: a graph's from its offsets[0] on
   uint32_t max_n = 0;
   std::vector<uint64_t> firsts;
   bool whole = false;  // union ids in the arenas (else every graph counts from 0)
@@ -241,7 +242,7 @@ __global__ void k_batch_in_off(uint64_t m, uint32_t n, const uint32_t* dst, uint
 // The union's in-edges, for the bottom-up levels: a stable sort by
 // destination, so in-lists stay in source order.
 static int batch_in_edges(gg_graph_batch_s* b, uint32_t n) {
-  const uint64_t m = b->total_m;
+  const uint64_t m = b->edges;
   GG_CUDA(cudaMalloc(&b->d_ioff, 4 * ((uint64_t)n + 1)));
   GG_CUDA(cudaMalloc(&b->d_iidx, 4 * (m + 16)));
   GG_CUDA(cudaMemsetAsync(b->d_iidx + m, 0, 64, b->stream));
@@ -286,16 +287,19 @@ static int batch_build(int32_t count, const gg_host_graph* graphs, gg_graph_batc
   std::vector<BatchDesc> desc(count);
   for (int32_t i = 0; i < count; ++i) {
     const gg_host_graph& h = graphs[i];
-    if (h.n == 0 || !h.offsets || (h.m && !h.indices) || h.offsets[h.n] != h.m)
+    if (h.n == 0 || !h.offsets || (h.m && !h.indices) || h.offsets[h.n] != h.m || h.offsets[0] > h.m)
       return fail(GG_ERR_INVALID_ARG, "gg_batch_create: graph %d is malformed", i);
     b->firsts.push_back(b->total_n);
     b->total_m += h.m;
     b->total_n += h.n;
     b->max_n = std::max(b->max_n, h.n);
   }
-  b->whole = b->total_n < (1ull << 31) && b->total_m < (1ull << 32) - 64;
+  // a graph's first edges, where offsets[0] is not 0, belong to no vertex and
+  // stay out of the arena
   std::vector<uint64_t> edge_first(count + 1, 0);
-  for (int32_t i = 0; i < count; ++i) edge_first[i + 1] = edge_first[i] + graphs[i].m;
+  for (int32_t i = 0; i < count; ++i) edge_first[i + 1] = edge_first[i] + graphs[i].m - graphs[i].offsets[0];
+  b->edges = edge_first[count];
+  b->whole = b->total_n < (1ull << 31) && b->edges < (1ull << 32) - 64;
   for (int32_t i = 0; i < count; ++i) {
     const uint64_t v0 = b->firsts[i];
     desc[i] = b->whole ? BatchDesc{v0, 0, v0, graphs[i].n, (uint32_t)v0}
@@ -306,7 +310,7 @@ static int batch_build(int32_t count, const gg_host_graph* graphs, gg_graph_batc
   GG_CUDA(cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking));
   GG_CUDA(cudaDeviceGetAttribute(&b->num_sms, cudaDevAttrMultiProcessorCount, b->device));
   GG_CUDA(cudaMalloc(&b->d_off, 4 * offs));
-  GG_CUDA(cudaMalloc(&b->d_idx, 4 * std::max<uint64_t>(b->total_m, 1)));
+  GG_CUDA(cudaMalloc(&b->d_idx, 4 * std::max<uint64_t>(b->edges, 1)));
   GG_CUDA(cudaMalloc(&b->d_levels, 4 * b->total_n));
   GG_CUDA(cudaMalloc(&b->d_desc, sizeof(BatchDesc) * count));
   GG_CUDA(cudaMalloc(&b->d_order, 4 * count));
@@ -318,15 +322,17 @@ static int batch_build(int32_t count, const gg_host_graph* graphs, gg_graph_batc
 #pragma omp parallel for schedule(dynamic, 8)
     for (int32_t i = 0; i < count; ++i) {
       const gg_host_graph& h = graphs[i];
-      const uint32_t base = b->whole ? (uint32_t)edge_first[i] : 0u;
+      const uint32_t base = (b->whole ? (uint32_t)edge_first[i] : 0u) - h.offsets[0];
       for (uint64_t v = 0; v < (uint64_t)h.n + (b->whole ? 0 : 1); ++v) off[desc[i].off_base + v] = h.offsets[v] + base;
     }
-    if (b->whole) off[b->total_n] = (uint32_t)b->total_m;
+    if (b->whole) off[b->total_n] = (uint32_t)b->edges;
     GG_TRY(upload(b, b->d_off, off.data(), offs));
     GG_CUDA(cudaStreamSynchronize(b->stream));  // off leaves scope
   }
   for (int32_t i = 0; i < count; ++i)
-    if (graphs[i].m) GG_TRY(upload<uint32_t>(b, b->d_idx + edge_first[i], graphs[i].indices, graphs[i].m));
+    if (edge_first[i + 1] > edge_first[i])
+      GG_TRY(upload<uint32_t>(b, b->d_idx + edge_first[i], graphs[i].indices + graphs[i].offsets[0],
+                              edge_first[i + 1] - edge_first[i]));
   if (b->whole) {
     uint64_t* d_first = nullptr;
     GG_CUDA(cudaMalloc(&d_first, 8 * ((uint64_t)count + 1)));
@@ -341,7 +347,7 @@ static int batch_build(int32_t count, const gg_host_graph* graphs, gg_graph_batc
     b->uni.idx = b->d_idx;
     b->uni.levels = b->d_levels;
     b->uni.n = (uint32_t)b->total_n;
-    b->uni.m = b->total_m;
+    b->uni.m = b->edges;
     // a batch whose in-edges or loop buffers do not fit beside it keeps one
     // CTA per graph
     b->loop = batch_in_edges(b, (uint32_t)b->total_n) == GG_OK;

@@ -1,5 +1,7 @@
 """Batches right after their creation: the copies of the host arrays, the
 kernels that renumber them and the first traversal are one sequence."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -24,3 +26,29 @@ def test_first_traversal_after_creation(gg, orc, count):
         b = gg.GraphBatch(hgs)
         check(gg, orc, hgs, b)
         b.close()
+
+
+class Late:
+    """hg with `lead` more entries before its first edge: offsets[0] = lead."""
+
+    def __init__(self, gg, hg, lead):
+        self.hg = hg
+        self.offsets = hg.offsets + np.uint32(lead)
+        self.indices = np.concatenate([np.full(lead, hg.n - 1, np.uint32), hg.indices])
+        p = C.POINTER(C.c_uint32)
+        self.c = gg.HostGraphC(hg.n, len(self.indices), 0, gg.W_NONE, self.offsets.ctypes.data_as(p),
+                               self.indices.ctypes.data_as(p), None)
+
+
+@pytest.mark.parametrize("leads", [(5, 0, 0), (0, 7, 300), (1, 1, 1)])
+def test_offsets_that_start_late(gg, orc, leads):
+    hgs = [gg.HostGraph.rmat(9, 8, seed=i, symmetric=False) for i in range(len(leads))]
+    late = [Late(gg, h, k) for h, k in zip(hgs, leads)]
+    b = gg.GraphBatch(late)
+    assert b.total_edges == sum(h.m for h in hgs) + sum(leads)
+    check(gg, orc, hgs, b)
+    b.close()
+    late[0].c.offsets[0] = late[0].c.m + 1
+    with pytest.raises(gg.GGError) as e:
+        gg.GraphBatch(late)
+    assert e.value.code == gg.ERR_INVALID_ARG
