@@ -316,6 +316,15 @@ static int batch_build(int32_t count, const gg_host_graph* graphs, gg_graph_batc
   GG_CUDA(cudaMalloc(&b->d_order, 4 * count));
   GG_CUDA(cudaMalloc(&b->d_src, 4 * count));
   GG_CUDA(cudaMalloc(&b->d_ctr, 16));
+  // all that one CTA per graph needs comes before the union's buffers, which a
+  // batch can do without
+  int per_sm = 0;
+  GG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batch_bfs, kBatchThreads, 0));
+  b->grid = std::max(1, std::min(count, b->num_sms * std::max(per_sm, 1)));
+  GG_CUDA(cudaMalloc(&b->d_scratch, 8ull * b->max_n * b->grid));
+  GG_CUDA(cudaMallocHost(&b->h_src, 4 * count));
+  GG_CUDA(cudaMallocHost(&b->h_levels, 4 * b->total_n));
+  GG_CUDA(cudaMallocHost(&b->h_ctr, 16 + sizeof(LoopState)));
   GG_TRY(upload(b, b->d_desc, desc.data(), count));
   {
     std::vector<uint32_t> off(offs);
@@ -367,13 +376,6 @@ static int batch_build(int32_t count, const gg_host_graph* graphs, gg_graph_batc
   std::stable_sort(order.begin(), order.end(), [&](uint32_t x, uint32_t y) { return graphs[x].m > graphs[y].m; });
   GG_TRY(upload(b, b->d_order, order.data(), count));
   GG_CUDA(cudaStreamSynchronize(b->stream));  // the host arrays are the caller's and this function's
-  int per_sm = 0;
-  GG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batch_bfs, kBatchThreads, 0));
-  b->grid = std::max(1, std::min(count, b->num_sms * std::max(per_sm, 1)));
-  GG_CUDA(cudaMalloc(&b->d_scratch, 8ull * b->max_n * b->grid));
-  GG_CUDA(cudaMallocHost(&b->h_src, 4 * count));
-  GG_CUDA(cudaMallocHost(&b->h_levels, 4 * b->total_n));
-  GG_CUDA(cudaMallocHost(&b->h_ctr, 16 + sizeof(LoopState)));
   // the replayed sequence: sources up, counters reset, traversal, counters down
   GG_CUDA(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
   cudaMemcpyAsync(b->d_src, b->h_src, 4 * count, cudaMemcpyHostToDevice, b->stream);
