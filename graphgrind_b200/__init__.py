@@ -40,6 +40,7 @@ BALANCE_EDGE, BALANCE_VERTEX = 0, 1
 PART_DEST, PART_SOURCE = 0, 1
 ORDER_CSR, ORDER_HILBERT = 0, 1
 VORDER_GIVEN, VORDER_HOT_FIRST = 0, 1
+BATCH_AUTO, BATCH_PER_CTA, BATCH_SEPARATE = 0, 1, 2
 EM_FORCE_SPARSE, EM_FORCE_CSC, EM_FORCE_COO, EM_NO_OUTPUT = 0x1, 0x2, 0x4, 0x8
 F_BFS, F_CC, F_PR, F_PRDELTA, F_SPMV, F_BF, F_BC, F_BC_BACK, F_BP = range(1, 10)
 
@@ -95,6 +96,10 @@ class EdgeMapStats(C.Structure):
     _fields_ = [("kind", C.c_int32), ("frontier_active", C.c_uint64),
                 ("frontier_out_edges", C.c_uint64), ("output_active", C.c_uint64),
                 ("output_out_edges", C.c_uint64)]
+
+
+class BatchOpts(C.Structure):
+    _fields_ = [("form", C.c_int32)]
 
 
 class Profile(C.Structure):
@@ -208,6 +213,7 @@ _sig("gg_ppr_k", C.c_int, _P, C.c_int32, C.c_int32, C.c_float, _P, _P, _P, C.POI
 _sig("gg_msbfs", C.c_int, _P, C.c_int32, _P, _P, C.POINTER(RunStats))
 _sig("gg_msbc", C.c_int, _P, C.c_int32, _P, _P, _P, C.POINTER(RunStats))
 _sig("gg_batch_create", C.c_int, C.c_int32, _P, C.POINTER(_P))
+_sig("gg_batch_create_opts", C.c_int, C.c_int32, _P, C.POINTER(BatchOpts), C.POINTER(_P))
 _sig("gg_batch_destroy", C.c_int, _P)
 _sig("gg_batch_info", C.c_int, _P, C.POINTER(C.c_uint64), C.POINTER(C.c_uint64), _P)
 _sig("gg_batch_bfs", C.c_int, _P, _P, _P, C.POINTER(RunStats))
@@ -234,7 +240,7 @@ EXPORTED = [
     "gg_vertex_array_free", "gg_memcpy_h2d", "gg_memcpy_d2h", "gg_host_alloc_pinned", "gg_host_free_pinned", "gg_bfs", "gg_components",
     "gg_pagerank", "gg_pagerank_delta", "gg_spmv", "gg_bellman_ford", "gg_bc", "gg_bp",
     "gg_bfs_push_step_noalloc", "gg_ppr_k", "gg_pagerank_converge", "gg_vebo", "gg_msbfs", "gg_msbc",
-    "gg_batch_create", "gg_batch_destroy", "gg_batch_info", "gg_batch_bfs",
+    "gg_batch_create", "gg_batch_create_opts", "gg_batch_destroy", "gg_batch_info", "gg_batch_bfs",
     "gg_pagerank_weighted_create", "gg_pagerank_weighted_destroy", "gg_pagerank_weighted_fwd",
     "gg_pagerank_weighted_bwd", "gg_autotune", "gg_autotune_build", "gg_autotune_ppr_k",
     "gg_hot_first_order", "gg_graph_vertex_order", "gg_host_graph_read_gpu", "gg_graph_device_weights",
@@ -765,13 +771,13 @@ def version() -> str:
 
 
 class GraphBatch:
-    """Many independent graphs in one device arena (gg_batch_*)."""
+    """Many independent graphs in one device arena (gg_batch_*); form: a gg_batch_form."""
 
-    def __init__(self, host_graphs):
+    def __init__(self, host_graphs, form=BATCH_AUTO):
         arr = (HostGraphC * len(host_graphs))(*[hg.c for hg in host_graphs])
         self._hosts = list(host_graphs)
         h = _P()
-        check(lib.gg_batch_create(len(host_graphs), arr, C.byref(h)), "gg_batch_create")
+        check(lib.gg_batch_create_opts(len(host_graphs), arr, C.byref(BatchOpts(form)), C.byref(h)), "gg_batch_create")
         self.h = h
         self.count = len(host_graphs)
         tn, tm = C.c_uint64(), C.c_uint64()

@@ -282,7 +282,7 @@ static int upload(gg_graph_batch_s* b, T* dst, const T* src, uint64_t count) {
   return GG_OK;
 }
 
-static int batch_build(int32_t count, const gg_host_graph* graphs, gg_graph_batch_s* b) {
+static int batch_build(int32_t count, const gg_host_graph* graphs, const gg_batch_opts& opts, gg_graph_batch_s* b) {
   b->count = count;
   std::vector<BatchDesc> desc(count);
   for (int32_t i = 0; i < count; ++i) {
@@ -299,7 +299,7 @@ static int batch_build(int32_t count, const gg_host_graph* graphs, gg_graph_batc
   std::vector<uint64_t> edge_first(count + 1, 0);
   for (int32_t i = 0; i < count; ++i) edge_first[i + 1] = edge_first[i] + graphs[i].m - graphs[i].offsets[0];
   b->edges = edge_first[count];
-  b->whole = b->total_n < (1ull << 31) && b->edges < (1ull << 32) - 64;
+  b->whole = opts.form != GG_BATCH_SEPARATE && b->total_n < (1ull << 31) && b->edges < (1ull << 32) - 64;
   for (int32_t i = 0; i < count; ++i) {
     const uint64_t v0 = b->firsts[i];
     desc[i] = b->whole ? BatchDesc{v0, 0, v0, graphs[i].n, (uint32_t)v0}
@@ -358,13 +358,17 @@ static int batch_build(int32_t count, const gg_host_graph* graphs, gg_graph_batc
     b->uni.n = (uint32_t)b->total_n;
     b->uni.m = b->edges;
     // a batch whose in-edges or loop buffers do not fit beside it keeps one
-    // CTA per graph
-    b->loop = batch_in_edges(b, (uint32_t)b->total_n) == GG_OK;
-    b->uni.ioff = b->d_ioff;
-    b->uni.iidx = b->d_iidx;
-    b->loop = b->loop && union_bfs_prepare(b->uni, b->device, b->num_sms) == GG_OK;
+    // CTA per graph, as on a device without cooperative launches
+    int rc = GG_ERR_UNSUPPORTED;
+    if (opts.form == GG_BATCH_AUTO) {
+      rc = batch_in_edges(b, (uint32_t)b->total_n);
+      b->uni.ioff = b->d_ioff;
+      b->uni.iidx = b->d_iidx;
+      if (!rc) rc = union_bfs_prepare(b->uni, b->device, b->num_sms);
+      if (rc && cudaGetLastError() != cudaErrorMemoryAllocation && rc != GG_ERR_UNSUPPORTED) return rc;
+    }
+    b->loop = rc == GG_OK;
     if (!b->loop) {
-      cudaGetLastError();
       union_bfs_free(b->uni);
       cudaFree(b->d_ioff);
       cudaFree(b->d_iidx);
@@ -411,7 +415,13 @@ using namespace gg;
 extern "C" {
 
 int gg_batch_create(int32_t count, const gg_host_graph* graphs, gg_graph_batch_t* out) {
-  if (count <= 0 || !graphs || !out) return fail(GG_ERR_INVALID_ARG, "gg_batch_create: bad arguments");
+  return gg_batch_create_opts(count, graphs, nullptr, out);
+}
+
+int gg_batch_create_opts(int32_t count, const gg_host_graph* graphs, const gg_batch_opts* opts, gg_graph_batch_t* out) {
+  const gg_batch_opts o = opts ? *opts : gg_batch_opts{GG_BATCH_AUTO};
+  if (count <= 0 || !graphs || !out || o.form < GG_BATCH_AUTO || o.form > GG_BATCH_SEPARATE)
+    return fail(GG_ERR_INVALID_ARG, "gg_batch_create: bad arguments");
   int devs = 0;
   if (cudaGetDeviceCount(&devs) != cudaSuccess || devs == 0) {
     cudaGetLastError();
@@ -419,7 +429,7 @@ int gg_batch_create(int32_t count, const gg_host_graph* graphs, gg_graph_batch_t
   }
   gg_graph_batch_s* b = new (std::nothrow) gg_graph_batch_s;
   if (!b) return fail(GG_ERR_OOM, "batch: out of host memory");
-  const int rc = batch_build(count, graphs, b);
+  const int rc = batch_build(count, graphs, o, b);
   if (rc) {
     const std::string keep = last_error();
     cudaStreamEndCapture(b->stream, &b->graph);  // leaves no capture open on a failed build

@@ -599,6 +599,16 @@ int gg_msbc(gg_graph_t g, int32_t k, const uint32_t* sources, float* dependencie
 typedef struct gg_graph_batch_s* gg_graph_batch_t;
 /* Uploads `count` host graphs (out-edge CSR each; weights ignored). */
 int gg_batch_create(int32_t count, const gg_host_graph* graphs, gg_graph_batch_t* out);
+/* How gg_batch_bfs runs: GG_BATCH_AUTO as described there; the other two are
+ * the forms it falls back to, for tests: GG_BATCH_PER_CTA one CTA per graph
+ * alone (a batch whose in-edges do not fit beside it), GG_BATCH_SEPARATE the
+ * same with every graph numbered from 0 (one past the union's size). */
+enum gg_batch_form { GG_BATCH_AUTO = 0, GG_BATCH_PER_CTA = 1, GG_BATCH_SEPARATE = 2 };
+typedef struct gg_batch_opts {
+  int32_t form; /* gg_batch_form */
+} gg_batch_opts;
+/* gg_batch_create with options (NULL: the defaults). */
+int gg_batch_create_opts(int32_t count, const gg_host_graph* graphs, const gg_batch_opts* opts, gg_graph_batch_t* out);
 int gg_batch_destroy(gg_graph_batch_t b);
 /* Sum of vertices and edges over the batch; firsts[count] (may be NULL)
  * receives each graph's first slot in the level output. */
