@@ -99,7 +99,7 @@ class EdgeMapStats(C.Structure):
 
 
 class BatchOpts(C.Structure):
-    _fields_ = [("form", C.c_int32)]
+    _fields_ = [("form", C.c_int32), ("wait_budget", C.c_int32)]
 
 
 class Profile(C.Structure):
@@ -771,13 +771,14 @@ def version() -> str:
 
 
 class GraphBatch:
-    """Many independent graphs in one device arena (gg_batch_*); form: a gg_batch_form."""
+    """Many independent graphs in one device arena (gg_batch_*); form: a gg_batch_form;
+    wait_budget: as in gg_batch_opts."""
 
-    def __init__(self, host_graphs, form=BATCH_AUTO):
+    def __init__(self, host_graphs, form=BATCH_AUTO, wait_budget=0):
         arr = (HostGraphC * len(host_graphs))(*[hg.c for hg in host_graphs])
         self._hosts = list(host_graphs)
         h = _P()
-        check(lib.gg_batch_create_opts(len(host_graphs), arr, C.byref(BatchOpts(form)), C.byref(h)), "gg_batch_create")
+        check(lib.gg_batch_create_opts(len(host_graphs), arr, C.byref(BatchOpts(form, wait_budget)), C.byref(h)), "gg_batch_create")
         self.h = h
         self.count = len(host_graphs)
         tn, tm = C.c_uint64(), C.c_uint64()

@@ -952,7 +952,7 @@ int union_bfs_enqueue(const UnionBfs& u, cudaStream_t s, int num_sms, const uint
   uint32_t ws = b.wstride, nn = u.n;
   int32_t round0 = 1, cap = u.n < (uint32_t)INT32_MAX ? (int32_t)u.n + 1 : INT32_MAX;
   unsigned long long thr = u.m / 20;  // edgeMap's m/20, over the union
-  unsigned budget = kWaitBudget;
+  unsigned budget = u.wait_budget;
   int vec = 1, mark = 1;
   // A level of the whole GPU costs about 10 us, a level inside one CTA per
   // graph about 2.5 us a window: below a window of edges per graph the second

@@ -41,6 +41,7 @@ struct UnionBfs {
   uint32_t* arena = nullptr;
   LoopState* st = nullptr;
   int grid = 0;
+  unsigned wait_budget = kWaitBudget;  // probes of a grid barrier's wait
 };
 // Allocates u's buffers for its n and m; union_bfs_free releases them.
 int union_bfs_prepare(UnionBfs& u, int device, int num_sms);

@@ -273,6 +273,17 @@ static int batch_in_edges(gg_graph_batch_s* b, uint32_t n) {
   return GG_OK;
 }
 
+// One CTA per graph, and its counters to the host: alone (st null), or from
+// where the union loop with state st stopped.
+static int batch_per_cta(gg_graph_batch_s* b, const LoopState* st) {
+  GG_CUDA(cudaMemsetAsync(b->d_ctr, 0, 16, b->stream));
+  k_batch_bfs<<<b->grid, kBatchThreads, 0, b->stream>>>(b->d_desc, b->d_order, b->count, b->d_off, b->d_idx,
+                                                          b->d_levels, b->d_src, b->d_ctr, b->d_scratch, b->max_n, st);
+  GG_CUDA(cudaGetLastError());
+  GG_CUDA(cudaMemcpyAsync(b->h_ctr, b->d_ctr, 16, cudaMemcpyDeviceToHost, b->stream));
+  return GG_OK;
+}
+
 // Host data to the device in the order of the batch's stream.  That stream does
 // not wait for the default stream, in which a plain copy of pageable memory may
 // still be under way when the call returns.
@@ -357,6 +368,7 @@ static int batch_build(int32_t count, const gg_host_graph* graphs, const gg_batc
     b->uni.levels = b->d_levels;
     b->uni.n = (uint32_t)b->total_n;
     b->uni.m = b->edges;
+    if (opts.wait_budget) b->uni.wait_budget = opts.wait_budget < 0 ? 0u : (unsigned)opts.wait_budget;
     // a batch whose in-edges or loop buffers do not fit beside it keeps one
     // CTA per graph, as on a device without cooperative launches
     int rc = GG_ERR_UNSUPPORTED;
@@ -383,12 +395,8 @@ static int batch_build(int32_t count, const gg_host_graph* graphs, const gg_batc
   // the replayed sequence: sources up, counters reset, traversal, counters down
   GG_CUDA(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
   cudaMemcpyAsync(b->d_src, b->h_src, 4 * count, cudaMemcpyHostToDevice, b->stream);
-  cudaMemsetAsync(b->d_ctr, 0, 16, b->stream);
   if (b->loop) GG_TRY(union_bfs_enqueue(b->uni, b->stream, b->num_sms, b->d_src, (uint32_t)count));
-  k_batch_bfs<<<b->grid, kBatchThreads, 0, b->stream>>>(b->d_desc, b->d_order, count, b->d_off, b->d_idx,
-                                                          b->d_levels, b->d_src, b->d_ctr, b->d_scratch, b->max_n,
-                                                          b->loop ? b->uni.st : nullptr);
-  cudaMemcpyAsync(b->h_ctr, b->d_ctr, 16, cudaMemcpyDeviceToHost, b->stream);
+  GG_TRY(batch_per_cta(b, b->loop ? b->uni.st : nullptr));
   if (b->loop)
     cudaMemcpyAsync(b->h_ctr + 2, b->uni.st, sizeof(LoopState), cudaMemcpyDeviceToHost, b->stream);
   GG_CUDA(cudaStreamEndCapture(b->stream, &b->graph));
@@ -419,7 +427,7 @@ int gg_batch_create(int32_t count, const gg_host_graph* graphs, gg_graph_batch_t
 }
 
 int gg_batch_create_opts(int32_t count, const gg_host_graph* graphs, const gg_batch_opts* opts, gg_graph_batch_t* out) {
-  const gg_batch_opts o = opts ? *opts : gg_batch_opts{GG_BATCH_AUTO};
+  const gg_batch_opts o = opts ? *opts : gg_batch_opts{GG_BATCH_AUTO, 0};
   if (count <= 0 || !graphs || !out || o.form < GG_BATCH_AUTO || o.form > GG_BATCH_SEPARATE)
     return fail(GG_ERR_INVALID_ARG, "gg_batch_create: bad arguments");
   int devs = 0;
@@ -475,19 +483,27 @@ int gg_batch_bfs(gg_graph_batch_t b, const uint32_t* sources, int32_t* levels, g
   GG_CUDA(cudaGraphLaunch(b->exec, b->stream));
   int32_t* down = levels && pinned_range(levels, 4 * b->total_n) ? levels : b->h_levels;
   GG_CUDA(cudaMemcpyAsync(down, b->d_levels, 4 * b->total_n, cudaMemcpyDeviceToHost, b->stream));
-  const double ms = tm.stop();
+  double ms = tm.stop();
   GG_CUDA(cudaStreamSynchronize(b->stream));
+  const LoopState* loop = b->loop ? reinterpret_cast<const LoopState*>(b->h_ctr + 2) : nullptr;
+  int kernels = loop ? 4 : 1;
+  uint64_t trav = loop ? loop->trav : 0;
+  if (loop && loop->exit_reason != 1 && loop->exit_reason != 4) {
+    // a grid barrier's wait ran out: one CTA per graph has none
+    GG_TRY(batch_per_cta(b, nullptr));
+    GG_CUDA(cudaMemcpyAsync(down, b->d_levels, 4 * b->total_n, cudaMemcpyDeviceToHost, b->stream));
+    ms = tm.stop();
+    GG_CUDA(cudaStreamSynchronize(b->stream));
+    ++kernels;
+    trav = 0;
+  }
   GG_CUDA(cudaGetLastError());
-  const LoopState* loop = reinterpret_cast<const LoopState*>(b->h_ctr + 2);
-  if (b->loop && loop->exit_reason < 0) return fail(GG_ERR_TIMEOUT, "gg_batch_bfs: a grid barrier wait ran out");
-  if (b->loop && loop->exit_reason != 1 && loop->exit_reason != 4)
-    return fail(GG_ERR_CUDA, "gg_batch_bfs: stopped without an empty frontier (reason %d)", loop->exit_reason);
   if (levels && down != levels) std::copy(b->h_levels, b->h_levels + b->total_n, levels);
   if (st) {
     st->ms = ms;
     st->rounds = 1;
-    st->edges_traversed = b->h_ctr[1] + (b->loop ? loop->trav : 0);
-    st->kernels = b->loop ? 4 : 1;
+    st->edges_traversed = trav + b->h_ctr[1];
+    st->kernels = kernels;
   }
   return GG_OK;
 }

@@ -605,7 +605,8 @@ int gg_batch_create(int32_t count, const gg_host_graph* graphs, gg_graph_batch_t
  * same with every graph numbered from 0 (one past the union's size). */
 enum gg_batch_form { GG_BATCH_AUTO = 0, GG_BATCH_PER_CTA = 1, GG_BATCH_SEPARATE = 2 };
 typedef struct gg_batch_opts {
-  int32_t form; /* gg_batch_form */
+  int32_t form;        /* gg_batch_form */
+  int32_t wait_budget; /* probes of the loop's grid-barrier waits; 0: the default, 2^22; < 0: none (for tests) */
 } gg_batch_opts;
 /* gg_batch_create with options (NULL: the defaults). */
 int gg_batch_create_opts(int32_t count, const gg_host_graph* graphs, const gg_batch_opts* opts, gg_graph_batch_t* out);
@@ -619,7 +620,8 @@ int gg_batch_info(gg_graph_batch_t b, uint64_t* total_vertices, uint64_t* total_
  * first, from a device work queue and finish each inside the CTA (a batch past
  * 2^31 vertices or 2^32 edges runs in that form alone).  levels: host array of
  * total_vertices int32 (may be NULL), graph i's at firsts[i], -1 unreached;
- * page-locked memory is filled without staging.  The sequence source upload ->
+ * page-locked memory is filled without staging.  Where a barrier wait of the
+ * whole-GPU levels runs out, the batch runs again with one CTA per graph.  The sequence source upload ->
  * traversal is a CUDA graph captured at gg_batch_create and replayed by every
  * call; st->ms is its device time with the level download, st->edges_traversed
  * the sum over graphs of gg_bfs's count. */

@@ -39,3 +39,24 @@ def test_unknown_form(gg, form):
     with pytest.raises(gg.GGError) as e:
         gg.GraphBatch([edgeless(gg, 3)], form)
     assert e.value.code == gg.ERR_INVALID_ARG
+
+
+@pytest.mark.parametrize("pinned", [False, True])
+def test_barrier_timeout_runs_without_barriers(gg, orc, pinned):
+    """With no probe at all, the CTAs that reach the first grid barrier before
+    the last one return at once; the call then gives the result all the same."""
+    hgs = [gg.HostGraph.rmat(15, 16, seed=3), gg.HostGraph.rmat(12, 16, seed=4, symmetric=False), edgeless(gg, 40)]
+    b = gg.GraphBatch(hgs, wait_budget=-1)
+    keep = gg.PinnedArray(b.total_vertices, np.int32)
+    out = keep.array if pinned else np.empty(b.total_vertices, np.int32)
+    for s in (0, 7, 0):
+        out[:] = -7
+        _, run = b.bfs(np.full(3, s, np.uint32), out)
+        assert run.kernels == 5
+        trav = 0
+        for h, lv in zip(hgs, b.split(out)):
+            _, olev, ost = orc.Graph.from_host(h).bfs(s)
+            np.testing.assert_array_equal(lv, olev)
+            trav += ost.edges_traversed
+        assert run.edges_traversed == trav
+    b.close()
