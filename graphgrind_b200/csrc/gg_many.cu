@@ -482,7 +482,13 @@ int gg_batch_bfs(gg_graph_batch_t b, const uint32_t* sources, int32_t* levels, g
   EventTimer tm(b->stream);
   GG_CUDA(cudaGraphLaunch(b->exec, b->stream));
   int32_t* down = levels && pinned_range(levels, 4 * b->total_n) ? levels : b->h_levels;
-  GG_CUDA(cudaMemcpyAsync(down, b->d_levels, 4 * b->total_n, cudaMemcpyDeviceToHost, b->stream));
+  cudaError_t copied = cudaMemcpyAsync(down, b->d_levels, 4 * b->total_n, cudaMemcpyDeviceToHost, b->stream);
+  if (copied == cudaErrorInvalidValue && down == levels) {  // page-locked at its ends only
+    cudaGetLastError();
+    down = b->h_levels;
+    copied = cudaMemcpyAsync(down, b->d_levels, 4 * b->total_n, cudaMemcpyDeviceToHost, b->stream);
+  }
+  GG_CUDA(copied);
   double ms = tm.stop();
   GG_CUDA(cudaStreamSynchronize(b->stream));
   const LoopState* loop = b->loop ? reinterpret_cast<const LoopState*>(b->h_ctr + 2) : nullptr;
