@@ -52,3 +52,19 @@ def test_offsets_that_start_late(gg, orc, leads):
     with pytest.raises(gg.GGError) as e:
         gg.GraphBatch(late)
     assert e.value.code == gg.ERR_INVALID_ARG
+
+
+def test_runs_of_vertices_without_in_edges(gg, orc):
+    """In-lists at the ends of long empty runs: before the first edge, between
+    two, behind the last, and graphs with none at all."""
+    def fan(n, u, dst):
+        off = np.zeros(n + 1, np.uint32)
+        off[u + 1:] = len(dst)
+        return gg.HostGraph.from_csr(off, np.array(dst, np.uint32))
+    n = 70_001
+    none = gg.HostGraph.from_csr(np.zeros(n + 1, np.uint32), np.zeros(0, np.uint32))
+    every = np.arange(0, n, 3)  # a first level dense enough for the bottom-up walk
+    hgs = [none, fan(n, n // 2, [n - 1]), fan(n, n // 2, [0, n - 1]), none, fan(n, n // 2, every), none]
+    b = gg.GraphBatch(hgs)
+    check(gg, orc, hgs, b)
+    b.close()
