@@ -618,7 +618,8 @@ int gg_batch_info(gg_graph_batch_t b, uint64_t* total_vertices, uint64_t* total_
  * as one union graph whose levels run on the whole GPU, top-down or bottom-up;
  * once the frontier is small, persistent CTAs take whole graphs, largest
  * first, from a device work queue and finish each inside the CTA (a batch past
- * 2^31 vertices or 2^32 edges runs in that form alone).  levels: host array of
+ * 2^31 vertices or 2^32 - 64 edges runs in that form alone, as does one of small
+ * graphs that are all resident at once).  levels: host array of
  * total_vertices int32 (may be NULL), graph i's at firsts[i], -1 unreached;
  * page-locked memory is filled without staging.  Where a barrier wait of the
  * whole-GPU levels runs out, the batch runs again with one CTA per graph.  The sequence source upload ->

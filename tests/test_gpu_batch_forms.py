@@ -60,3 +60,16 @@ def test_barrier_timeout_runs_without_barriers(gg, orc, pinned):
             trav += ost.edges_traversed
         assert run.edges_traversed == trav
     b.close()
+
+
+@pytest.mark.parametrize("n,kernels", [(3072, 1), (3073, 4)])
+def test_small_graphs_skip_the_union(gg, orc, n, kernels):
+    """n vertices in a path: n + m = 2 n - 1, on both sides of 6144."""
+    off = np.minimum(np.arange(n + 1), n - 1).astype(np.uint32)
+    hgs = [gg.HostGraph.from_csr(off, np.arange(1, n, dtype=np.uint32)), edgeless(gg, 5)]
+    b = gg.GraphBatch(hgs)
+    lev, run = b.bfs([n - 40, 2])
+    assert run.kernels == kernels
+    for h, s, lv in zip(hgs, (n - 40, 2), b.split(lev)):
+        np.testing.assert_array_equal(lv, orc.Graph.from_host(h).bfs(s)[1])
+    b.close()
