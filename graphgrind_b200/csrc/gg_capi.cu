@@ -325,6 +325,14 @@ static int run_bfs(gg_graph_s* g, uint32_t start, int32_t* parents, int32_t* lev
     GG_TRY(edge_map(g, F.f, f, thr, 0, &out));
     F.reset(out);
   }
+  // the loop's outcome goes to the host before the device work that the loop
+  // feeds: the host sees it while that work runs
+  Event outcome;
+  if (full) {
+    GG_TRY(bfs_device_full_begin_result(g));
+    GG_CUDA(cudaEventCreateWithFlags(&outcome.e, cudaEventDisableTiming));
+    GG_CUDA(cudaEventRecord(outcome.e, g->stream));
+  }
   const int32_t* par_out = par;
   const int32_t* lev_out = lev;
   const int pslot = g->async_results && g->ws.d_order[2] ? 2 : 0;  // the given-order array of the parents
@@ -339,15 +347,13 @@ static int run_bfs(gg_graph_s* g, uint32_t start, int32_t* parents, int32_t* lev
   if (parents && !g->relabeled) GG_TRY(given_order<int32_t>(g, par, pslot, &par_out));
   if (levels) GG_TRY(given_order<int32_t>(g, lev, 1, &lev_out));
   tm.mark();
-  // the all-levels launch is read back after the device work it feeds and the
-  // copies of its results were queued behind it: one wait for all of them
-  if (full) GG_TRY(bfs_device_full_begin_result(g));
-  GG_TRY(to_host(g, parents, par_out, n));
-  GG_TRY(to_host(g, levels, lev_out, n));
+  // only a finished traversal is written to the caller's arrays
   if (full) {
-    GG_CUDA(cudaStreamSynchronize(g->stream));
+    GG_CUDA(cudaEventSynchronize(outcome.e));
     GG_TRY(bfs_device_full_result(g, &round, &trav));
   }
+  GG_TRY(to_host(g, parents, par_out, n));
+  GG_TRY(to_host(g, levels, lev_out, n));
   fill_stats(st, tm.elapsed(), round, trav, g->kernels);
   return GG_OK;
 }

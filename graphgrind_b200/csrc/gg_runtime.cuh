@@ -41,6 +41,14 @@ struct EventTimer {
   }
 };
 
+// An event of one call.
+struct Event {
+  cudaEvent_t e = nullptr;
+  ~Event() {
+    if (e) cudaEventDestroy(e);
+  }
+};
+
 // Stream-ordered allocations of the library (temporaries of the
 // applications, frontiers) come from one memory pool per device whose release
 // threshold is unlimited: memory freed back to it stays mapped across stream
