@@ -78,12 +78,30 @@ __device__ __forceinline__ bool grid_barrier(unsigned* bar, unsigned target, uns
   return *s_ok != 0;
 }
 
-// A queue slot whose edges start at eoff notes itself as the first slot of
-// every window whose first edge it holds, so that a CTA finds its window's
-// slots with one load.
+// A queue slot whose edges start at eoff is noted as the first slot of every
+// window whose first edge it holds, so that a CTA finds its window's slots with
+// one load.
 __device__ __forceinline__ void note_windows(uint32_t* wst, uint32_t slot, uint32_t eoff, uint32_t deg) {
   for (uint64_t w = ((uint64_t)eoff + kLoopThreads - 1) / kLoopThreads; w * kLoopThreads < (uint64_t)eoff + deg; ++w)
     wst[w] = slot;
+}
+// The same for the lanes of a warp that add a slot (every lane calls it): a
+// lane notes the first windows itself, and the warp a hub's others (a star's hub
+// of 16M out-edges, 32768 windows: traversal 0.33 ms with one lane's stores, 0.18
+// now).
+constexpr uint32_t kOwnWindows = 256, kHubEdges = kOwnWindows * kLoopThreads;
+__device__ __forceinline__ void note_windows_warp(uint32_t* wst, bool add, uint32_t slot, uint32_t eoff, uint32_t deg) {
+  const uint32_t w0 = (uint32_t)(((uint64_t)eoff + kLoopThreads - 1) / kLoopThreads);
+  const uint32_t w1 = add ? (uint32_t)(((uint64_t)eoff + deg + kLoopThreads - 1) / kLoopThreads) : w0;
+  for (uint32_t w = w0; w < w1 && w - w0 < kOwnWindows; ++w) wst[w] = slot;
+  uint32_t hubs = __ballot_sync(0xffffffffu, w1 - w0 > kOwnWindows);
+  while (hubs) {
+    const int l = __ffs(hubs) - 1;
+    hubs &= hubs - 1;
+    const uint32_t b = __shfl_sync(0xffffffffu, w0, l) + kOwnWindows, e = __shfl_sync(0xffffffffu, w1, l);
+    const uint32_t sl = __shfl_sync(0xffffffffu, slot, l);
+    for (uint32_t w = b + (threadIdx.x & 31); w < e; w += 32) wst[w] = sl;
+  }
 }
 
 // Warp-cooperative append to the next frontier (every lane calls it).  A
@@ -109,12 +127,12 @@ __device__ __forceinline__ void loop_append(bool add, uint32_t u, uint32_t deg, 
     unsigned long long old = 0;
     if (lane == leader) old = atomicAdd(packed, ((unsigned long long)__popc(bal) << 32) | wsum);
     old = __shfl_sync(0xffffffffu, old, leader);
+    const uint32_t slot = (uint32_t)(old >> 32) + __popc(bal & lanemask_lt), eoff = (uint32_t)old + inc - deg;
     if (pos) {
-      const uint64_t slot = (old >> 32) + __popc(bal & lanemask_lt);
       nq[slot] = u;
-      neo[slot] = (uint32_t)old + inc - deg;
-      note_windows(nwst, (uint32_t)slot, (uint32_t)old + inc - deg, deg);
+      neo[slot] = eoff;
     }
+    note_windows_warp(nwst, pos, slot, eoff, deg);
   }
   const uint32_t zb = __ballot_sync(0xffffffffu, zer);
   if (zb) {
@@ -165,16 +183,17 @@ __device__ __forceinline__ void block_append(bool add, uint32_t u, uint32_t deg,
   if (threadIdx.x == 0 && np) s_base[0] = atomicAdd(packed, ((unsigned long long)np << 32) | (uint32_t)total);
   if (threadIdx.x == 32 && nz) s_base[1] = atomicAdd(zeros, (unsigned long long)nz);
   __syncthreads();
+  uint32_t slot = 0, eoff = 0;
   if (pos) {
     const unsigned long long old = s_base[0];
-    const uint32_t slot = (uint32_t)(old >> 32) + (uint32_t)(ex >> 48);
-    const uint32_t eoff = (uint32_t)old + (uint32_t)ex;
+    slot = (uint32_t)(old >> 32) + (uint32_t)(ex >> 48);
+    eoff = (uint32_t)old + (uint32_t)ex;
     nq[slot] = u;
     neo[slot] = eoff;
-    note_windows(nwst, slot, eoff, deg);
   } else if (zer) {
     nq[n - 1 - (s_base[1] + ((uint32_t)(ex >> 32) & 0xffffu))] = u;
   }
+  note_windows_warp(nwst, pos, slot, eoff, deg);
 }
 
 // The shared memory of a sparse level's window.
@@ -693,6 +712,7 @@ __global__ void __launch_bounds__(kLoopThreads, 2048 / kLoopThreads)
         const uint32_t w = c0 + tid;
         const uint32_t x = w < w1 ? bnxt[w] : 0u;
         uint32_t mp = 0, md = 0;
+        bool hub = false;
         uint32_t y = x;
         while (y) {
           const uint32_t v = w * 32 + (__ffs(y) - 1);
@@ -701,6 +721,7 @@ __global__ void __launch_bounds__(kLoopThreads, 2048 / kLoopThreads)
           if (d) {
             ++mp;
             md += d;
+            hub |= d > kHubEdges;
           }
         }
         // slots and edges of the words before (at most 32 kLoopThreads slots)
@@ -709,15 +730,33 @@ __global__ void __launch_bounds__(kLoopThreads, 2048 / kLoopThreads)
         __syncthreads();
         uint32_t slot = (uint32_t)base_p + (uint32_t)(ex >> 32), eoff = (uint32_t)base_d + (uint32_t)ex;
         y = x;
-        while (y) {
-          const uint32_t v = w * 32 + (__ffs(y) - 1);
-          y &= y - 1;
-          const uint32_t d = off[v + 1] - off[v];
-          if (d) {
-            nq[slot] = v;
-            neo[slot] = eoff;
-            note_windows(nwst, slot, eoff, d);
-            ++slot;
+        if (!__any_sync(0xffffffffu, hub)) {
+          while (y) {
+            const uint32_t v = w * 32 + (__ffs(y) - 1);
+            y &= y - 1;
+            const uint32_t d = off[v + 1] - off[v];
+            if (d) {
+              nq[slot] = v;
+              neo[slot] = eoff;
+              note_windows(nwst, slot, eoff, d);
+              ++slot;
+              eoff += d;
+            }
+          }
+        } else {
+          while (__any_sync(0xffffffffu, y != 0)) {
+            uint32_t d = 0;
+            if (y) {
+              const uint32_t v = w * 32 + (__ffs(y) - 1);
+              y &= y - 1;
+              d = off[v + 1] - off[v];
+              if (d) {
+                nq[slot] = v;
+                neo[slot] = eoff;
+              }
+            }
+            note_windows_warp(nwst, d != 0, slot, eoff, d);
+            slot += d != 0;
             eoff += d;
           }
         }
