@@ -186,10 +186,10 @@ struct gg_graph_s {
   gg::RoundLoop* round_loop[3] = {nullptr, nullptr, nullptr};  // BellmanFord, Components, PageRankDelta: created by their first call
   int round_graph = 1;  // dense COO rounds of BellmanFord / Components / PageRankDelta as a CUDA graph
   // GG_TUNE_EARLY_KERNEL 3's in-lists (the CSC's, each by descending source
-  // out-degree), built by the second all-levels BFS (m_pad entries): a graph
-  // traversed once does not pay for them
+  // out-degree; m_pad entries), built by the first all-levels BFS after the
+  // caller has set the knob to 3
   uint32_t* d_bu_idx = nullptr;
-  bool bfs_ran = false;
+  bool bu_wanted = false;
   int coo_kernel = 7;  // 0 CTA ring (k_pull), 1 per-warp direct loads, 2/3 per-warp bulk-copy rings, 6 direct loads
                        // with cross-lane run merging, 7 the same with cache hints (fastest measured)
   // gg_build_opts.vertex_order: device ids differ from the given ids

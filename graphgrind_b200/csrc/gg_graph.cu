@@ -1082,6 +1082,7 @@ int gg_graph_set_tuning(gg_graph_t g, int32_t key, int64_t value) {
     case GG_TUNE_EARLY_KERNEL:
       if (value < 0 || value > 3) return fail(GG_ERR_INVALID_ARG, "early-exit kernel must be 0..3");
       g->early_kernel = (int)value;
+      g->bu_wanted = value == 3;
       return GG_OK;
     case GG_TUNE_PUSH_DENSE_DIV:
       if (value < 0 || value > (1ll << 30)) return fail(GG_ERR_INVALID_ARG, "push-dense divisor must be 0..2^30");

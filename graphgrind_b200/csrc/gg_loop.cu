@@ -850,13 +850,15 @@ int bfs_device_full_prepare(gg_graph_s* g, bool want_levels, DevBuf<uint32_t>& a
   GG_TRY(full_bufs(g, want_levels, nullptr, &b));
   GG_TRY(arena.alloc(g, b.words));
   // the bottom-up levels walk the in-lists hub sources first (same edges,
-  // other order: a vertex then meets a frontier in-neighbour sooner)
-  // (graphs the copy cannot be built for, past 2^31 edges or without the
-  // memory, walk the CSC's own in-lists).  The copy costs a segmented sort of
-  // all edges and its temporaries (R-MAT-22: 17 ms against a traversal of
-  // 0.2 ms), so the first BFS of a graph walks the CSC's in-lists too.
-  if (g->early_kernel == 3 && !g->d_bu_idx && g->bfs_ran && build_bu_index(g) != GG_OK) cudaGetLastError();
-  g->bfs_ran = true;
+  // other order: a vertex then meets a frontier in-neighbour sooner), where the
+  // caller has asked for that copy (graphs it cannot be built for, past 2^31
+  // edges or without the memory, walk the CSC's own in-lists).  It is not built
+  // unasked: it costs a segmented sort of all edges and its temporaries, which
+  // takes thousands of traversals to earn back (17 ms on R-MAT-22 against a
+  // loop of 172 instead of 176 us, on R-MAT-24 433 instead of 447 us; on
+  // Erdos-Renyi graphs the loop is slower with it, 281 against 275 us).
+  if (g->bu_wanted && !g->d_bu_idx && build_bu_index(g) != GG_OK) cudaGetLastError();
+  g->bu_wanted = false;
   return GG_OK;
 }
 

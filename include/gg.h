@@ -416,15 +416,16 @@ int gg_graph_set_dense_policy(gg_graph_t g, int32_t policy);
  *                         frontier tests issued together (also in the
  *                         bottom-up levels of GG_TUNE_DEVICE_LOOP 2: BFS on
  *                         R-MAT-24 0.453 against 0.473 ms with 0); 3
- *                         (default) as 2, and the bottom-up levels of
- *                         GG_TUNE_DEVICE_LOOP 2 walk a copy of the in-lists
- *                         with each list's sources by descending out-degree
- *                         (a vertex meets a frontier in-neighbour sooner:
- *                         0.438 against 0.452 ms); the second such BFS builds
- *                         the copy (one segmented sort), which stays with the
- *                         graph: 4 bytes per edge (a graph past 2^31 edges,
- *                         or one the copy does not fit beside, walks the
- *                         CSC's own in-lists)
+ *                         (default) as 2; a program that sets it to 3 also
+ *                         has the bottom-up levels of GG_TUNE_DEVICE_LOOP 2
+ *                         walk a copy of the in-lists with each list's
+ *                         sources by descending out-degree (a vertex meets a
+ *                         frontier in-neighbour sooner: 0.433 against 0.447
+ *                         ms on R-MAT-24): the next such BFS builds the copy
+ *                         (one segmented sort: 17 ms on R-MAT-22), which
+ *                         stays with the graph: 4 bytes per edge (a graph
+ *                         past 2^31 edges, or one the copy does not fit
+ *                         beside, walks the CSC's own in-lists)
  *   GG_TUNE_PUSH_DENSE_DIV  a dense edgeMap of BFS (an early-exit functor)
  *                         whose frontier has at most n / value vertices runs
  *                         top-down instead (the frontier's out-edges pushed,
