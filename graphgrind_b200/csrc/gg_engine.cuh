@@ -142,12 +142,17 @@ struct gg_graph_s {
   gg::SegIndex seg[2];       // row structure of the pulled stream, same indexing
   uint64_t m_pad = 0;        // edge arrays hold m_pad entries (zero padded)
   gg::TileSet coo_tiles;
-  // work items of the direct-load COO pulls: two uint4 each, the tile and
-  // {first 256-edge block, blocks, items of the tile, slab word of the tile};
-  // a tile shared by several items combines their sums in its slab
-  uint4* d_coo_items = nullptr;
-  uint32_t coo_item_count = 0;
-  uint32_t* d_coo_slab = nullptr;  // all zero between launches
+  // work items of the direct-load COO pulls, of those with an output and of
+  // those without: two uint4 each, the tile and {first 256-edge block, blocks,
+  // items of the tile, slab word of the tile}; a tile shared by several items
+  // combines their sums in its slab
+  struct CooItems {
+    uint4* d = nullptr;
+    uint32_t count = 0;
+    bool split = false;  // some tile is shared by several
+  } coo_items[2];
+  uint4 *d_coo_whole = nullptr, *d_coo_cut = nullptr;  // the lists: whole tiles, cut ones (where used)
+  uint32_t* d_coo_slab = nullptr;                      // all zero between launches
   uint2* d_coo_gaps = nullptr;  // {first, count} of the destination ranges outside every COO tile
   uint32_t coo_gap_count = 0;
   bool has_coo = false;
@@ -247,7 +252,7 @@ struct PullParams {
   unsigned long long* stats;   // [0] count [1] out-degree sum
   unsigned long long* err;
   uint32_t tv;                 // widest tile of the tile set
-  const uint4* items;          // work items of the COO tiles (see gg_graph_s::d_coo_items)
+  const uint4* items;          // work items of the COO tiles (see gg_graph_s::coo_items)
   uint32_t nitems;
   uint32_t* slab;
 };
@@ -520,7 +525,7 @@ struct finishes<F, decltype((void)F::kFinish)> {
 
 constexpr int kCooWarps = 8;
 constexpr int kCooThreads = kCooWarps * 32;
-constexpr uint64_t kCooItemMinEdges = 4096;  // fewest edges a tile is cut into (build_coo_items)
+constexpr uint64_t kCooItemMinEdges = 12288;  // fewest edges a tile is cut into (build_coo_items)
 
 __host__ __device__ constexpr size_t coo_w_stage_bytes(bool hw) {
   return (size_t)kSegBlock * 4 + (size_t)kSegBlock * 2 + (hw ? (size_t)kSegBlock * 4 : 0);

@@ -375,50 +375,79 @@ int build_bu_index(gg_graph_s* g) {
   return GG_OK;
 }
 
-// Work items of the merging COO pulls (pull_coo_w_run).  An item aims at half
-// the edges a resident CTA takes on average (4 CTAs per SM), so that the last
-// CTAs finish together, but at no fewer than four edges per destination of the
-// tile: below that the passes over the tile's accumulators and its slab cost
-// more than the balance gains (PageRank pull, R-MAT-20 / R-MAT-22 with
-// 2^18-edge tiles: half an average share and 4 edges per destination 87.7 /
-// 218 us, a quarter and 2 edges 93.6 / 216 us, whole tiles 92 / 365 us).  A
-// tile of less than one and a half items stays whole.
-static int build_coo_items(gg_graph_s* g) {
-  const uint64_t per_cta = g->coo_len / ((uint64_t)g->num_sms * 4);
-  std::vector<uint4> items;
-  uint64_t slab = 0;
-  struct Part {
-    uint32_t tile, first, blocks, parts;
-    uint64_t slab;
+// A list of work items of the COO tiles, longest first: tile t in parts[t]
+// items, whose slab starts at word slab[t].
+static int upload_coo_items(gg_graph_s* g, const std::vector<uint32_t>& parts, const std::vector<uint64_t>& slab,
+                            uint4** d, uint32_t* count) {
+  struct Item {
+    uint32_t tile, first, blocks;
   };
-  std::vector<Part> parts;
+  std::vector<Item> list;
   for (uint32_t t = 0; t < g->coo_tiles.count; ++t) {
-    const uint4 td = g->coo_tiles.host[t];
-    const uint32_t nb = (td.w + kSegBlock - 1) / kSegBlock;
-    const uint64_t want = std::max<uint64_t>({per_cta / 2, 4ull * td.y, kCooItemMinEdges});
-    const uint32_t k = (uint32_t)std::min<uint64_t>(nb, std::max<uint64_t>(1, (td.w + want / 2) / want));
+    const uint32_t nb = (g->coo_tiles.host[t].w + kSegBlock - 1) / kSegBlock;
     uint32_t b = 0;
-    for (uint32_t i = 0; i < k; ++i) {
-      const uint32_t e = (uint32_t)((uint64_t)nb * (i + 1) / k);
-      parts.push_back(Part{t, b, e - b, k, slab});
+    for (uint32_t i = 0; i < parts[t]; ++i) {
+      const uint32_t e = (uint32_t)((uint64_t)nb * (i + 1) / parts[t]);
+      list.push_back(Item{t, b, e - b});
       b = e;
     }
-    if (k > 1) slab += 4 + ((td.y + 3) & ~3u) + ((td.y + 127) / 128) * 4;
   }
-  if (slab >= (1ull << 32)) return fail(GG_ERR_SIZE, "COO slabs exceed 2^32 words");
-  std::stable_sort(parts.begin(), parts.end(), [](const Part& a, const Part& b) { return a.blocks > b.blocks; });
-  for (const Part& q : parts) {
+  std::stable_sort(list.begin(), list.end(), [](const Item& a, const Item& b) { return a.blocks > b.blocks; });
+  std::vector<uint4> items;
+  for (const Item& q : list) {
     items.push_back(g->coo_tiles.host[q.tile]);
-    items.push_back(make_uint4(q.first, q.blocks, q.parts, (uint32_t)q.slab));
+    items.push_back(make_uint4(q.first, q.blocks, parts[q.tile], (uint32_t)slab[q.tile]));
   }
-  g->coo_item_count = (uint32_t)parts.size();
-  GG_TRY(dev_alloc(g, &g->d_coo_items, std::max<size_t>(items.size(), 1)));
-  if (!items.empty())
-    GG_CUDA(cudaMemcpy(g->d_coo_items, items.data(), sizeof(uint4) * items.size(), cudaMemcpyHostToDevice));
-  if (slab) {
-    GG_TRY(dev_alloc(g, &g->d_coo_slab, slab));
-    GG_CUDA(cudaMemset(g->d_coo_slab, 0, 4 * slab));
+  *count = (uint32_t)list.size();
+  GG_TRY(dev_alloc(g, d, std::max<size_t>(items.size(), 1)));
+  if (!items.empty()) GG_CUDA(cudaMemcpy(*d, items.data(), sizeof(uint4) * items.size(), cudaMemcpyHostToDevice));
+  return GG_OK;
+}
+
+// Work items of the merging COO pulls (pull_coo_w_run).  Cutting a tile costs
+// the passes over its accumulators and its slab once per item, and every CTA
+// the joining code's registers, so tiles are cut only on graphs whose largest
+// tile outlasts the others: one above twice the edges a resident CTA takes on
+// average (4 CTAs per SM).  CTAs of an SM share its load pipe, so up to there a
+// long tile speeds up once its neighbours are done (Erdos-Renyi, 384 tiles of
+// 1.54 shares: PageRank 1040 us whole, 1165 cut; R-MAT-22, 0.9: 2550 / 2600;
+// R-MAT-20, 2.4: 1030 / 850; R-MAT-22 with 2^18-edge tiles, 2.4: 4260 / 2590).
+// Steps without an output join cheaper, and are cut from one and a half shares
+// (the 1.54 above: SpMV 148 us whole, 139 cut).  An item aims at half a share,
+// at no fewer than four edges per destination of the tile and no fewer than
+// kCooItemMinEdges (R-MAT-18, 103 tiles of up to 64K edges: 595 us with 8192,
+// 565 with 12288, 530 with 16384; R-MAT-20: 856, 852, 1007).  A tile of less
+// than two items stays whole: cut in two, it would leave the ones just below it
+// as the longest (Erdos-Renyi, 128 tiles of up to 24840 edges, items of 16384:
+// 484 us with those rounded up to two items, 411 whole).
+static int build_coo_items(gg_graph_s* g) {
+  const uint64_t per_cta = g->coo_len / ((uint64_t)g->num_sms * 4);
+  const uint32_t tiles = g->coo_tiles.count;
+  std::vector<uint32_t> whole(tiles, 1), cut(tiles, 1);
+  std::vector<uint64_t> slab(tiles, 0);
+  uint64_t words = 0, largest = 0;
+  for (uint32_t t = 0; t < tiles; ++t) {
+    const uint4 td = g->coo_tiles.host[t];
+    const uint64_t want = std::max<uint64_t>({per_cta / 2, 4ull * td.y, kCooItemMinEdges});
+    cut[t] = (uint32_t)std::max<uint64_t>(1, td.w / want);
+    slab[t] = words;
+    if (cut[t] > 1) words += 4 + ((td.y + 3) & ~3u) + ((td.y + 127) / 128) * 4;
+    largest = std::max<uint64_t>(largest, td.w);
   }
+  const bool cut_any = words > 0 && 2 * largest > 3 * per_cta, cut_all = cut_any && largest > 2 * per_cta;
+  if (cut_any && words >= (1ull << 32)) return fail(GG_ERR_SIZE, "COO slabs exceed 2^32 words");
+  gg_graph_s::CooItems lists[2];
+  if (!cut_all) GG_TRY(upload_coo_items(g, whole, slab, &g->d_coo_whole, &lists[0].count));
+  lists[0].d = g->d_coo_whole;
+  if (cut_any) {
+    GG_TRY(upload_coo_items(g, cut, slab, &g->d_coo_cut, &lists[1].count));
+    lists[1].d = g->d_coo_cut;
+    lists[1].split = true;
+    GG_TRY(dev_alloc(g, &g->d_coo_slab, words));
+    GG_CUDA(cudaMemset(g->d_coo_slab, 0, 4 * words));
+  }
+  g->coo_items[0] = lists[cut_all];
+  g->coo_items[1] = lists[cut_any];
   return GG_OK;
 }
 
@@ -713,7 +742,8 @@ static void graph_release(gg_graph_s* g) {
     cudaFree(s.d_rows);
   }
   cudaFree(g->coo_tiles.d_tiles);
-  cudaFree(g->d_coo_items);
+  cudaFree(g->d_coo_whole);
+  cudaFree(g->d_coo_cut);
   cudaFree(g->d_coo_slab);
   cudaFree(g->d_coo_gaps);
   cudaFree(g->d_coo_src);

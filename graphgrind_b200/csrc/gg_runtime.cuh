@@ -311,8 +311,8 @@ int pull_launch(gg_graph_s* g, gg_frontier_s* in, gg_frontier_s* out, const F& f
     p.dloc = g->d_coo_dloc;
     p.wts = g->d_coo_w;
     p.off = nullptr;
-    p.items = g->d_coo_items;
-    p.nitems = g->coo_item_count;
+    p.items = g->coo_items[no_out].d;
+    p.nitems = g->coo_items[no_out].count;
     p.slab = g->d_coo_slab;
   } else {
     p.tiles = g->csc_tiles[orient].d_tiles;
@@ -358,7 +358,7 @@ int pull_launch(gg_graph_s* g, gg_frontier_s* in, gg_frontier_s* out, const F& f
     static DeviceOnce opted[2][4];
     static DeviceOnce opted_pf[2];
     static DeviceOnce opted_no[4][2];
-    const bool split = g->d_coo_slab != nullptr;  // some tile is cut into several work items
+    const bool split = g->coo_items[no_out].split;
     static DeviceOnce opted_mg[2];
     constexpr int kFlags = coo_w_flag_bytes<F, false>(), kFlagsNoOut = coo_w_flag_bytes<F, true>();
     auto launch_w = [&](auto kern, int stages, DeviceOnce& once, int flags) -> int {
