@@ -47,6 +47,7 @@ static bool wpr_live(const gg_wpr_s* w) {
 // Sums into S: rows inside a block are stored, rows split across blocks added.
 struct SumInto {
   using T = float;
+  static constexpr bool kMayScan = false;
   float* S;
   __device__ static T identity() { return 0.f; }
   __device__ static T combine(T a, T b) { return a + b; }

@@ -23,7 +23,7 @@ __device__ __forceinline__ void atomic_mul(float* a, float b) {
 
 struct BpOp {
   using T = float2;
-  static constexpr bool kNeedsIdx = false, kNeedsRow = true;
+  static constexpr bool kNeedsIdx = false, kNeedsRow = true, kMayScan = true;
   const float2* vp;   // [n] vertex potentials
   const float4* ep;   // [m] edge potentials, (i, k) at component 2 i + k
   const float2* cur;  // [n] products of the previous iteration

@@ -96,6 +96,7 @@ struct SegIndex {
   uint32_t* d_blk = nullptr;
   uint32_t* d_rows = nullptr;
   uint64_t nrows = 0;
+  uint32_t longest = 0;  // edges of the longest row
 };
 
 // Size of Workspace::h_map, the largest control block read back through it.

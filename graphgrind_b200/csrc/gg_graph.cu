@@ -233,6 +233,7 @@ static int build_seg(gg_graph_s* g, const uint32_t* off, SegIndex& si) {
   for (uint32_t v = 0; v < n; ++v) {
     if (off[v + 1] == off[v]) continue;
     const uint32_t e = off[v];
+    si.longest = std::max(si.longest, off[v + 1] - e);
     head[e >> 5] |= 1u << (e & 31);
     blk[e / kSegBlock + 1]++;
     rows.push_back(v);
