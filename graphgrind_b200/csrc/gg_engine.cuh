@@ -1761,7 +1761,12 @@ __global__ void __launch_bounds__(kPushThreads) k_push_bits(const PushParams p, 
 // CTAs (with 4096 edges per CTA, a step of 100K edges ran 16 windows deep on 25
 // CTAs: 29 us, now 8), a CTA finds its first queue slot by 256-way search
 // rounds, stages the slots of its window in shared memory, and appends with
-// one atomic.
+// one atomic.  A CTA's windows follow one another, so the staged slots also tell
+// where the next window starts (grid of 1000^2, all vertices active: 132 us with
+// a search per window, 115).  A window ends when its slowest atomic has
+// returned, so destinations whose bit is already set are left out of the
+// atomics on the dedup words, where an R-MAT graph's hubs meet (R-MAT-20, all
+// 16M edges: 920 us with them, 491).
 template <class F, bool HW>
 __global__ void __launch_bounds__(kPushThreads) k_push(const PushParams p, const F f) {
   __shared__ uint32_t s_off[kPushThreads], s_q[kPushThreads], s_beg[kPushThreads];
@@ -1775,12 +1780,13 @@ __global__ void __launch_bounds__(kPushThreads) k_push(const PushParams p, const
   const uint64_t per = (windows + gridDim.x - 1) / gridDim.x;
   const uint64_t w1 = windows < (blockIdx.x + 1) * per ? windows : (blockIdx.x + 1) * per;
   uint32_t scur = 0;
+  bool search = p.k > kPushThreads;  // a queue of one stage is staged whole
   for (uint64_t w = blockIdx.x * per; w < w1; ++w) {
     const uint32_t base = (uint32_t)(w * kPushThreads);
     const uint32_t last = (uint32_t)(E < (w + 1) * kPushThreads ? E - 1 : (w + 1) * kPushThreads - 1);
     // the slot that holds the window's first edge: the last one whose offset
-    // is at most that (a queue of one stage is staged whole)
-    if (p.k > kPushThreads) {
+    // is at most that
+    if (search) {
       uint32_t lo = scur, hi = p.k;
       while (hi - lo > 1) {
         const uint32_t step = (hi - lo + kPushThreads - 1) / kPushThreads;
@@ -1803,7 +1809,9 @@ __global__ void __launch_bounds__(kPushThreads) k_push(const PushParams p, const
     const int ns = __syncthreads_count(mine);
     // vertices without out-edges take slots but no edges, so the window may
     // reach past the staged slots; its threads then search the queue itself
-    const bool past = ns == kPushThreads && (uint64_t)scur + ns < p.k && p.offs[scur + ns] <= last;
+    const bool more = (uint64_t)scur + kPushThreads < p.k;
+    const uint32_t after = ns < kPushThreads ? s_off[ns] : more ? p.offs[scur + kPushThreads] : 0xffffffffu;
+    const bool past = after <= last;
     const uint32_t e = base + tid;
     bool take = false;
     uint32_t d = 0;
@@ -1828,10 +1836,9 @@ __global__ void __launch_bounds__(kPushThreads) k_push(const PushParams p, const
       }
       d = p.idx[ei];
       const uint32_t wt = HW ? p.wts[ei] : 1u;
-      if (f.cond(d) && f.update_atomic(s, d, wt)) {
-        const uint32_t bit = 1u << (d & 31);
-        take = !(atomicOr(p.dedup + (d >> 5), bit) & bit);
-      }
+      // (loaded beside the update)
+      const uint32_t seen = __ldcg(p.dedup + (d >> 5)), bit = 1u << (d & 31);
+      if (f.cond(d) && f.update_atomic(s, d, wt) && !(seen & bit)) take = !(atomicOr(p.dedup + (d >> 5), bit) & bit);
     }
     const uint32_t ball = __ballot_sync(0xffffffffu, take);
     if (lane == 0) s_cnt[warp] = __popc(ball);
@@ -1847,6 +1854,12 @@ __global__ void __launch_bounds__(kPushThreads) k_push(const PushParams p, const
     if (take) {
       p.out_q[s_base + before + __popc(ball & ((1u << lane) - 1u))] = d;
       my_deg += p.deg_off[d + 1] - p.deg_off[d];
+    }
+    // the next window's first edge is the first one of the slot after the
+    // staged ones, or else the last staged slot's
+    if (p.k > kPushThreads) {
+      search = past;
+      if (!past) scur += ns - (after != last + 1);
     }
   }
   my_deg = warp_sum(my_deg);
