@@ -871,6 +871,8 @@ struct RoundLoopCtl {
   unsigned long long trav;       // out-degree sums of the inputs of the rounds after the first
   unsigned long long dm;         // next frontier: members
   unsigned long long out_edges;  //   and their out-degree sum
+  unsigned long long in_dm;      // the last round's input: members
+  unsigned long long in_edges;   //   and their out-degree sum
   unsigned long long err;        // device error word seen by a check
   double l1;                     // PageRankDelta: L1 of the last round
   double eps;                    //   and its stop threshold
@@ -948,10 +950,13 @@ __global__ void k_round_check(RoundLoopCtl* c, unsigned long long* stats, unsign
   } else {
     const long long fm = (long long)dm, tot = (long long)oe;
     const bool pull = tot > 0 && fm + tot > c->threshold && (c->coo_always || fm + tot > c->dense_threshold);
-    if (pull)
+    if (pull) {
       c->trav += oe;
-    else
+      c->in_dm = dm;
+      c->in_edges = oe;
+    } else {
       reason = 3;
+    }
   }
   c->reason = reason;
   cudaGraphSetConditional(h_loop, reason == 0 ? 1u : 0u);
@@ -1129,6 +1134,8 @@ static int round_loop_run(gg_graph_s* g, RoundLoop* L, FrontierHold& F, uint32_t
   c.coo_always = dense_takes_coo(g) || !(g->dense_policy == 0 || g->transposed) ? 1u : 0u;
   c.use_l1 = l1 ? 1u : 0u;
   c.eps = eps;
+  c.in_dm = in->dm;
+  c.in_edges = in->out_edges;
   GG_TRY(write_small(g, L->d_ctl, c));
   GG_CUDA(cudaGraphLaunch(L->exec, g->stream));
   GG_TRY(read_small(g, L->h_ctl, L->d_ctl));
@@ -1139,8 +1146,12 @@ static int round_loop_run(gg_graph_s* g, RoundLoop* L, FrontierHold& F, uint32_t
   *trav += in->out_edges + c.trav;
   if (l1) *l1 = c.l1;
   g->kernels += L->per_round * (int)c.count;
+  // the last round, as edge_map reports it: its kind is the rule's, not the kernel's
+  const bool ref_rule = g->dense_policy == 0 || g->transposed;
   g->last = gg_edge_map_stats{};
-  g->last.kind = 3;
+  g->last.kind = ref_rule && (long long)(c.in_dm + c.in_edges) <= c.dense_threshold ? 2 : 3;
+  g->last.frontier_active = c.in_dm;
+  g->last.frontier_out_edges = c.in_edges;
   g->last.output_active = c.dm;
   g->last.output_out_edges = c.out_edges;
   gg_frontier_s* o = nullptr;
