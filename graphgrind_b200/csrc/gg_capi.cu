@@ -129,13 +129,13 @@ __global__ void k_pr_epilogue(uint32_t n, int all, const uint32_t* fbits, float*
 // 73-105 and 158-165): the vertexFilter over all vertices (PR_Vertex_F, in the
 // first round PR_Vertex_F_FirstRound) into out_bits with its count and
 // out-degree sum, L1 = sum |Delta|, nghSum reset to 0 and the next round's
-// contrib = Delta/outdeg.  It moves 32 bytes per vertex; the counts take one
-// atomic per CTA (a filter with one per warp and a separate epilogue took 18
-// us on R-MAT-20, this 8).
+// contrib = Delta/outdeg, the only form in which Delta is read again.  It moves
+// 24 bytes per vertex; the counts take one atomic per CTA (a filter with one
+// per warp and a separate epilogue took 18 us on R-MAT-20, this 8).
 template <bool FIRST>
-__global__ void __launch_bounds__(256) k_prd_vertex(uint32_t n, float* p, float* delta, float* ngh,
-                                                    const uint32_t* __restrict__ off, float* contrib, uint32_t* out_bits, unsigned long long* stats,
-                                                    double* l1, float damping, float added, float one_over_n,
+__global__ void __launch_bounds__(256) k_prd_vertex(uint32_t n, float* p, float* ngh, const uint32_t* __restrict__ off,
+                                                    float* contrib, uint32_t* out_bits,
+                                                    unsigned long long* stats, double* l1, float damping, float added, float one_over_n,
                                                     float eps2) {
   constexpr int U = 2;  // 32-vertex groups in flight per warp
   __shared__ unsigned long long s_sum[2][8];
@@ -174,7 +174,6 @@ __global__ void __launch_bounds__(256) k_prd_vertex(uint32_t n, float* p, float*
           pi = pv[u] + d;
         }
         p[v] = pi;
-        delta[v] = d;
         ngh[v] = 0.0f;
         contrib[v] = dg[u] ? d / (float)dg[u] : 0.0f;
         acc += fabsf(d);
@@ -202,11 +201,11 @@ __global__ void __launch_bounds__(256) k_prd_vertex(uint32_t n, float* p, float*
 }
 
 template <bool FIRST>
-static int prd_vertex(gg_graph_s* g, float* p, float* delta, float* ngh, float* contrib, uint32_t* out_bits,
+static int prd_vertex(gg_graph_s* g, float* p, float* ngh, float* contrib, uint32_t* out_bits,
                       unsigned long long* stats) {
   const double n = (double)g->n;
   k_prd_vertex<FIRST><<<generic_grid(g, g->n), kGenericThreads, 0, g->stream>>>(
-      g->n, p, delta, ngh, g->out_off(), contrib, out_bits, stats, g->ws.d_red, 0.85f, (float)((1 - 0.85) * (1 / n)),
+      g->n, p, ngh, g->out_off(), contrib, out_bits, stats, g->ws.d_red, 0.85f, (float)((1 - 0.85) * (1 / n)),
       (float)(1 / n), 0.01f);
   GG_CUDA(cudaGetLastError());
   g->kernels++;
@@ -888,7 +887,7 @@ struct RoundLoopCtl {
 
 struct RoundLoop {
   // BellmanFord: distances, Visited; Components: IDs, prevIDs; PageRankDelta:
-  // p, Delta, nghSum, contributions (n + 4 entries of 4 bytes each)
+  // p, Delta (of the start), nghSum, contributions (n + 4 entries of 4 bytes each)
   void* arr[4] = {nullptr, nullptr, nullptr, nullptr};
   uint32_t* bits[3] = {nullptr, nullptr, nullptr};  // frontiers of the rounds (0, 1); PageRankDelta's pull output (2)
   unsigned long long* d_fstats = nullptr;  // PageRankDelta: the vertexFilter's count and out-degree sum
@@ -1006,7 +1005,6 @@ static int round_launches(gg_graph_s* g, RoundLoop* L, int app, uint32_t* in_bit
   // PageRankDelta: the pull's output (discarded by the application) into the
   // third bitmap, the vertexFilter over all vertices into out_bits
   float* p = static_cast<float*>(L->arr[0]);
-  float* delta = static_cast<float*>(L->arr[1]);
   float* ngh = static_cast<float*>(L->arr[2]);
   float* contrib = static_cast<float*>(L->arr[3]);
   out.d_bits = L->bits[2];
@@ -1014,7 +1012,7 @@ static int round_launches(gg_graph_s* g, RoundLoop* L, int app, uint32_t* in_bit
   f.contrib = contrib;
   f.acc_out = ngh;
   GG_TRY((pull_launch<PrF, false>(g, &in, &out, f, true)));
-  return prd_vertex<false>(g, p, delta, ngh, contrib, out_bits, L->d_fstats);
+  return prd_vertex<false>(g, p, ngh, contrib, out_bits, L->d_fstats);
 }
 
 static int round_loop_capture(gg_graph_s* g, RoundLoop* L, int app) {
@@ -1452,8 +1450,8 @@ static int run_pagerank_delta(gg_graph_s* g, float* ranks, gg_run_stats* st) {
     GG_TRY(frontier_ensure_bits(A.f, false));
     GG_TRY(reset_stats(g));
     GG_CUDA(cudaMemsetAsync(g->ws.d_red, 0, sizeof(double), g->stream));
-    GG_TRY(round == 1 ? prd_vertex<true>(g, p, delta, ngh, contrib, A.f->d_bits, g->ws.d_stats)
-                      : prd_vertex<false>(g, p, delta, ngh, contrib, A.f->d_bits, g->ws.d_stats));
+    GG_TRY(round == 1 ? prd_vertex<true>(g, p, ngh, contrib, A.f->d_bits, g->ws.d_stats)
+                      : prd_vertex<false>(g, p, ngh, contrib, A.f->d_bits, g->ws.d_stats));
     double l1;
     GG_TRY(read_stats_red(g, &l1));
     A.f->has_dense = true;
