@@ -1085,7 +1085,7 @@ static RoundLoop* round_loop_get(gg_graph_s* g, int app) {
     for (int i = 0; i < nb; ++i) ok = ok && cudaMalloc((void**)&L->bits[i], bb) == cudaSuccess;
     if (app == kRoundLoopPrd) {
       ok = ok && cudaMalloc((void**)&L->d_fstats, 4 * sizeof(unsigned long long)) == cudaSuccess;
-      ok = ok && cudaMemset(L->d_fstats, 0, 4 * sizeof(unsigned long long)) == cudaSuccess;
+      ok = ok && cudaMemsetAsync(L->d_fstats, 0, 4 * sizeof(unsigned long long), g->stream) == cudaSuccess;
     }
     ok = ok && cudaMalloc((void**)&L->d_ctl, sizeof(RoundLoopCtl)) == cudaSuccess;
     ok = ok && cudaMallocHost((void**)&L->h_ctl, sizeof(RoundLoopCtl)) == cudaSuccess;

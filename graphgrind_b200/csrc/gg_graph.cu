@@ -1384,6 +1384,7 @@ int gg_vertex_array_free(gg_graph_t g, void* p) {
 }
 int gg_memcpy_h2d(void* d, const void* h, size_t bytes) {
   GG_CUDA(cudaMemcpy(d, h, bytes, cudaMemcpyHostToDevice));
+  GG_CUDA(cudaStreamSynchronize(nullptr));  // the graphs' streams do not wait for a copy of pageable memory
   return GG_OK;
 }
 int gg_memcpy_d2h(void* h, const void* d, size_t bytes) {
