@@ -135,8 +135,8 @@ __global__ void k_pr_epilogue(uint32_t n, int all, const uint32_t* fbits, float*
 template <bool FIRST>
 __global__ void __launch_bounds__(256) k_prd_vertex(uint32_t n, float* p, float* ngh, const uint32_t* __restrict__ off,
                                                     float* contrib, uint32_t* out_bits,
-                                                    unsigned long long* stats, double* l1, float damping, float added, float one_over_n,
-                                                    float eps2) {
+                                                    unsigned long long* stats, double* l1, float damping, float added,
+                                                    float one_over_n, float eps2) {
   constexpr int U = 2;  // 32-vertex groups in flight per warp
   __shared__ unsigned long long s_sum[2][8];
   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -856,9 +856,9 @@ static int pr_loop_get(gg_graph_s* g, bool bit_all, PrLoop** out) {
 // the next from 1 into 0.  A round is the application's edgeMap (the COO
 // pull, with its output count and out-degree sum) and its vertex step
 // (BellmanFord: Visited reset over the output; Components: prevIDs = IDs over
-// the input, before the pull; PageRankDelta: the vertexFilter over all
-// vertices, whose output is the next frontier, and the epilogue with the L1
-// norm; its pull's own output goes to a third bitmap nobody reads).  After
+// the input, before the pull; PageRankDelta: k_prd_vertex, the vertexFilter
+// over all vertices, whose output is the next frontier, with the L1 norm and
+// the next contributions; its pull's own output goes to a third bitmap nobody reads).  After
 // each round a check kernel counts it, clears the round's input bitmap (the
 // next output) and applies the host loop's tests: stop on an empty frontier,
 // at the round cap (BellmanFord's n rounds) or when L1 < eps
@@ -880,7 +880,7 @@ struct RoundLoopCtl {
   uint32_t count;                // rounds run
   uint32_t max_rounds;
   uint32_t reason;               // 0 running, 1 empty frontier or L1 < eps, 2 round cap, 3 handed back, 4 device error
-  uint32_t coo_always;           // the dense policy pins the COO pull (else the m/2 rule)
+  uint32_t coo_always;           // every dense round pulls over the COO (dense_takes_coo or the policy; else above m/2)
   uint32_t use_l1;               // stop on L1 < eps
   uint32_t pad;
 };

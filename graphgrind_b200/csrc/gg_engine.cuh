@@ -546,22 +546,6 @@ __host__ __device__ constexpr size_t coo_w_smem_bytes(bool hw, int stages, int v
 #ifndef GG_COO_MIN_BLOCKS
 #define GG_COO_MIN_BLOCKS 4  // resident CTAs per SM the register allocation must allow
 #endif
-// NOOUT: the caller discards edgeMap's output (GG_EM_NO_OUTPUT) and F's
-// commit of the identity is a no-op (sums): no touched flags, no next-frontier
-// bits, no stats; destinations with a non-identity sum are committed.
-// MERGE: destination runs that continue across lanes are combined with warp
-// shuffles before the shared-memory accumulation, so a destination appears in
-// at most one accumulation per block (instead of one per lane it spans, all
-// on one address).
-// The merging kernels (MERGE) take their work as items: a tile, or a run of
-// 256-edge blocks of one.  What bounds the pull is the L1/LSU pipe of the SMs
-// that still have edges: with one CTA per tile, an R-MAT hub tile (up to
-// tile_edges edges) outlasts every other CTA (R-MAT-22, 2^18-edge tiles, 65M
-// edges on 592 resident CTAs: 110K edges per CTA, 255K in the largest tile).
-// A tile's items add their sums to its slab in global memory (encoded so that
-// zero is the identity of every functor) and the item that arrives last takes
-// the totals back, clears the slab and commits, so that every destination is
-// still committed once.
 // The end of a work item of a tile cut into `items`: this item's sums and
 // touched marks go to the tile's slab, and the CTA that arrives last takes the
 // totals back into shared memory, clears the slab and returns true (to commit).
@@ -622,6 +606,22 @@ struct has_gather_pol : std::false_type {};
 template <class F>
 struct has_gather_pol<F, decltype((void)std::declval<const F&>().gather_pol(0u, 0u, 0ull))> : std::true_type {};
 
+// The COO pull, one CTA per tile or item.
+// NOOUT: the caller discards edgeMap's output (GG_EM_NO_OUTPUT) and F's
+// commit of the identity is a no-op (sums): no touched flags, no next-frontier
+// bits, no stats; destinations with a non-identity sum are committed.
+// MERGE: the last destination runs of a block's lanes are combined with warp
+// shuffles before the shared-memory accumulation, so that a destination
+// spanning many lanes does not put one accumulation per lane on one address.
+// The merging kernels take their work as items: a tile, or a run of 256-edge
+// blocks of one.  What bounds the pull is the L1/LSU pipe of the SMs that
+// still have edges: with one CTA per tile, an R-MAT hub tile (up to tile_edges
+// edges) outlasts every other CTA (R-MAT-22, 2^18-edge tiles, 65M edges on 592
+// resident CTAs: 110K edges per CTA, 255K in the largest tile).  A tile's items
+// add their sums to its slab in global memory (encoded so that zero is the
+// identity of every functor) and the item that arrives last takes the totals
+// back, clears the slab and commits, so that every destination is still
+// committed once.
 // HINT bits of the direct-load pull: 1 the edge stream bypasses L1 and is
 // marked evict-first in L2; 2 the source gathers (functors with gather_pol)
 // are marked evict-last in L1 and L2; 4 a vertex step at the commits
@@ -730,14 +730,18 @@ __device__ __forceinline__ void pull_coo_w_run(const PullParams& p, const F& f) 
     if constexpr (PF) {
       if (nbw > 0) pload(0);
     }
-    // One 256-edge block of a merging kernel.  What bounds the pull on graphs
-    // whose sources stay in L2 is the instruction issue, so the block is
-    // straight-line code: the edges are sorted by destination, a lane keeps one
+    // One 256-edge block of a merging kernel, as straight-line code, so that
+    // its loads and atomics are not held up by divergent loops (a third fewer
+    // instructions): the edges are sorted by destination, a lane keeps one
     // running value and passes it on where the next edge has another
-    // destination (predicated, no divergent loop), and the lanes' last runs
-    // are merged by a segmented scan, which a block whose lanes all end on
-    // different destinations skips.  FULL: every slot holds an edge (all blocks
-    // of a tile but its last), so nothing is tested per slot.
+    // destination (predicated), and the lanes' last runs are merged by a
+    // segmented scan, which a block whose lanes all end on different
+    // destinations skips.  FULL: every slot holds an edge (all blocks of a tile
+    // but its last), so nothing is tested per slot.  A lane's first run goes to
+    // shared memory by itself even where it continues the lane before: holding
+    // it back to join them costs more (PageRank pull on R-MAT-24 0.790 against
+    // 0.824 ms), except on R-MAT-21 and -22 in given order (2330 against 2290
+    // us and 2560 against 2515 for ten iterations).
     auto merge_block = [&](auto full, uint32_t j) {
       constexpr bool FULL = decltype(full)::value;
       constexpr bool kAllValid = FULL && ALL && F::kCondTrue;

@@ -658,7 +658,7 @@ __global__ void __launch_bounds__(kLoopThreads, 2048 / kLoopThreads)
     const unsigned long long npk = s_rd[0];
     const unsigned long long nk2 = nrep == 0 ? (npk >> 32) + s_rd[1] : s_rd[2];
     const unsigned long long nE = nrep == 0 ? npk & 0xffffffffull : s_rd[3];
-    // a frontier this small that no longer grows fast goes back to the caller
+    // a frontier this small that grows by less than four times goes back to the caller, for good
     const bool give = nk2 + nE < handover && nE < 4 * E;
     if (nk2 == 0 || give) {
       if (blockIdx.x == 0 && tid == 0) {

@@ -5,13 +5,15 @@
 // level's edges are spread over the GPU whatever graph they belong to, where
 // one CTA per graph would leave the GPU waiting for the largest one (256
 // R-MAT graphs of scale 10-16, 90M edges: 8.5 ms, of which the largest graph
-// alone).  Once the frontier is small and no longer grows, a persistent kernel
-// takes over, whose CTAs take whole graphs from a device work queue (largest
+// alone).  Once the frontier has fewer than a window of edges per graph and grows
+// by less than four times a level, a persistent kernel takes over, for the rest
+// of the traversal, whose CTAs take whole graphs from a device work queue (largest
 // first) and finish each inside the CTA without grid barriers: its
 // level-synchronous top-down traversal of app/BFS.C:77-101 balances a
 // frontier's edges over the CTA's threads by a block prefix sum over the
-// frontier's degrees.  Batches past 2^31 vertices or 2^32 edges, and those whose
-// in-edges do not fit beside them, run in that kernel alone.  The launch
+// frontier's degrees.  Batches past 2^31 vertices or 2^32 - 64 edges, those whose
+// in-edges do not fit beside them, and small graphs that are all resident at
+// once run in that kernel alone.  The launch
 // sequence is captured once as a CUDA graph and replayed.
 #include <cub/cub.cuh>
 

@@ -520,7 +520,8 @@ typedef struct gg_run_stats {
 } gg_run_stats;
 
 /* app/BFS.C:77-101: parents[n] (-1 unreached), levels[n] (-1 unreached); either
- * output may be NULL (app/BFS.C's result is the parents). */
+ * output may be NULL (app/BFS.C's result is the parents).  After an expired
+ * barrier wait (GG_ERR_TIMEOUT) both are as they were. */
 int gg_bfs(gg_graph_t g, uint32_t start, int32_t* parents, int32_t* levels, gg_run_stats* st);
 /* app/Components.C:101-126: ids[n]. */
 int gg_components(gg_graph_t g, int32_t* ids, gg_run_stats* st);
@@ -617,13 +618,14 @@ int gg_batch_destroy(gg_graph_batch_t b);
 int gg_batch_info(gg_graph_batch_t b, uint64_t* total_vertices, uint64_t* total_edges, uint64_t* firsts);
 /* BFS from sources[i] in graph i for every graph (app/BFS.C:77-101 levels),
  * as one union graph whose levels run on the whole GPU, top-down or bottom-up;
- * once the frontier is small, persistent CTAs take whole graphs, largest
- * first, from a device work queue and finish each inside the CTA (a batch past
- * 2^31 vertices or 2^32 - 64 edges runs in that form alone, as does one of small
- * graphs that are all resident at once).  levels: host array of
+ * once the frontier is small (fewer than 512 edges per graph, growing by less
+ * than four times a level), persistent CTAs take whole graphs, largest first,
+ * from a device work queue and finish each inside the CTA (a batch past 2^31
+ * vertices or 2^32 - 64 edges runs in that form alone, as does one of small
+ * graphs that are all resident at once; where a barrier wait of the whole-GPU
+ * levels runs out, the batch runs again in that form).  levels: host array of
  * total_vertices int32 (may be NULL), graph i's at firsts[i], -1 unreached;
- * page-locked memory is filled without staging.  Where a barrier wait of the
- * whole-GPU levels runs out, the batch runs again with one CTA per graph.  The sequence source upload ->
+ * page-locked memory is filled without staging.  The sequence source upload ->
  * traversal is a CUDA graph captured at gg_batch_create and replayed by every
  * call; st->ms is its device time with the level download, st->edges_traversed
  * the sum over graphs of gg_bfs's count. */
