@@ -324,14 +324,19 @@ static int run_bfs(gg_graph_s* g, uint32_t start, int32_t* parents, int32_t* lev
     GG_TRY(edge_map(g, F.f, f, thr, 0, &out));
     F.reset(out);
   }
-  // the loop's outcome goes to the host before the device work that the loop
-  // feeds: the host sees it while that work runs
+  // The loop's outcome goes to the host before the device work that the loop
+  // feeds, so that the host sees it while that work runs.  With asynchronous
+  // results it goes behind that work: results of earlier calls may be on their
+  // way, and its write to the host then waits for them (28 us of a BFS on
+  // R-MAT-24 after PageRank and SpMV).
   Event outcome;
-  if (full) {
+  auto read_outcome = [&]() -> int {
     GG_TRY(bfs_device_full_begin_result(g));
     GG_CUDA(cudaEventCreateWithFlags(&outcome.e, cudaEventDisableTiming));
     GG_CUDA(cudaEventRecord(outcome.e, g->stream));
-  }
+    return GG_OK;
+  };
+  if (full && !g->async_results) GG_TRY(read_outcome());
   const int32_t* par_out = par;
   const int32_t* lev_out = lev;
   const int pslot = g->async_results && g->ws.d_order[2] ? 2 : 0;  // the given-order array of the parents
@@ -348,6 +353,7 @@ static int run_bfs(gg_graph_s* g, uint32_t start, int32_t* parents, int32_t* lev
   tm.mark();
   // only a finished traversal is written to the caller's arrays
   if (full) {
+    if (g->async_results) GG_TRY(read_outcome());
     GG_CUDA(cudaEventSynchronize(outcome.e));
     GG_TRY(bfs_device_full_result(g, &round, &trav));
   }
